@@ -288,10 +288,14 @@ COUL_API int coul_forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n
  * least-squares loss L = 0.5 sum_i w_i (V_i - T_i)^2 pass G_i = w_i (V_i - T_i).  No counterpart in KTT
  * (it tunes forward kernels only); the PyTorch binding wraps forward + adjoint as an autograd function.
  * Asynchronous on the context's stream; keeps an FP64 workspace of 32 * n_atoms * chunks bytes in the
- * context (chunks ~ 24 * SMs / atom tiles).
+ * context (chunks <= 40 * SMs / atom tiles of 128).
  */
 COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
                              const float* d_grad_map, float* d_grad_q, float* d_grad_xyz);
+/* The same gradients as one n_atoms x 4 array (dL/dx, dL/dy, dL/dz, dL/dq), the layout of the atoms:
+   what the PyTorch binding returns, without a second pass to interleave them.  d_grad 16-byte aligned. */
+COUL_API int coul_adjoint_3d_packed(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
+                                    const float* d_grad_map, float* d_grad);
 
 /* ---- N-body: the sibling pair sum of KTT's Nbody example ---------------------------------- */
 /* Tuning fields (the KTT parameter each one covers in brackets, Examples/Nbody/Nbody.cpp:140-209). */

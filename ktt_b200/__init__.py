@@ -437,13 +437,11 @@ def adjoint_3d(ctx: "CoulombContext", atoms, dims, spacing, grad_map, origin=Non
     if g.numel() != nx * ny * nz or not g.is_cuda:
         raise CoulombError(COUL_ERR_INVALID_ARGUMENT, "grad_map must be a CUDA tensor with nx*ny*nz elements")
     n = atoms.shape[0]
-    grad_q = torch.empty(n, dtype=torch.float32, device=atoms.device)
-    grad_xyz = torch.empty((n, 3), dtype=torch.float32, device=atoms.device)
+    grad = torch.empty((n, 4), dtype=torch.float32, device=atoms.device)
     ctx._bind_stream()
     grid = _grid(dims, spacing, origin)
-    _check(ctx._lib.coul_adjoint_3d(ctx.handle, _ptr(atoms), n, ctypes.byref(grid), _ptr(g), _ptr(grad_q),
-                                    _ptr(grad_xyz)))
-    return torch.cat([grad_xyz, grad_q[:, None]], dim=1)
+    _check(ctx._lib.coul_adjoint_3d_packed(ctx.handle, _ptr(atoms), n, ctypes.byref(grid), _ptr(g), _ptr(grad)))
+    return grad
 
 
 def _autograd_function():

@@ -24,6 +24,7 @@ def register(lib) -> None:
         "coul_batch_info": [vp, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ci), ctypes.POINTER(ctypes.c_double)],
         "coul_pack_atoms": [vp, vp, vp, vp, vp, ctypes.c_int64, vp],
         "coul_adjoint_3d": [vp, vp, ctypes.c_int64, ctypes.POINTER(_Grid), vp, vp, vp],
+        "coul_adjoint_3d_packed": [vp, vp, ctypes.c_int64, ctypes.POINTER(_Grid), vp, vp],
         "coul_nbody_tune_default": [ctypes.POINTER(NbodyTuneC)],
         "coul_nbody_tune_supported": [ctypes.POINTER(NbodyTuneC)],
         "coul_nbody_step": [vp, vp, vp, ctypes.c_int64, ctypes.c_float, ctypes.c_float, ctypes.c_float,

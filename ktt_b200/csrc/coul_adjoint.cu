@@ -5,17 +5,20 @@
 //     dL/dq_j = sum_i G_i / r_ij
 //     dL/dr_j = q_j sum_i G_i (r_i - r_j) / r_ij^3
 // Nothing is stored per pair: 1/r is recomputed.  KTT has no adjoint; this is the B200 form of the
-// transposed sum.  Each CTA owns a tile of atoms (kAdjThreads threads x A atoms in registers) and a
-// chunk of grid rows; the rows' G values stream through shared memory in 256-point segments, stored
-// with the point's x coordinate as {G, G, x, x} so that one broadcast 16-byte shared load hands every
-// thread both operands already paired for the packed instructions (no per-point int-to-float
-// conversion, which would share the XU pipe with the rsqrts), and every thread evaluates each point
-// against its atoms.  Along a
-// row dy and dz are constant, so per pair the work is dx, r^2 = fma(dx, dx, dy^2 + dz^2), rsqrt,
-// t = G/r, accumulate t, t3 = t/r^2, accumulate t3*dx and t3 (the y and z components are dy and dz
-// times the row sum of t3): 8 FP32 operations and one MUFU rsqrt.  Row partials (FP32) go into FP64
-// per-atom accumulators; each (atom tile, row chunk) writes its FP64 partials, and a second kernel
-// adds the chunks in a fixed order, so the result is deterministic.
+// transposed sum.  A thread owns one atom, a CTA kAdjThreads atoms and a chunk of grid rows; the rows'
+// G values pass through shared memory in blocks of kRows rows x X points, and while a block of
+// X columns is processed the thread holds its X differences dx = x - a.x in registers, so a
+// pair costs six FP32 operations -- r^2 = fma(dx, dx, dy^2 + dz^2), 1/r^2, 1/r^3, and three FMAs that
+// add G/r (for the charge), G/r^3 by column (its sum times dx gives the x component) and G/r^3 by row
+// (its sum times dy and dz gives the other two) -- and one MUFU rsqrt.  Two neighbouring columns share
+// each packed instruction: dx, the column sums and the four-point loads of G come in pairs as they
+// are.  The FP32 sums of one block go into FP64 sums per atom; each (atom tile, row chunk) writes its
+// FP64 partials, and a second kernel adds the chunks in a fixed order, so the result is deterministic.
+//
+// Bound: the MUFU unit (one rsqrt a pair at 16 a clock and SM, 4.64e12 pairs/s; the six FP32
+// operations alone would allow 5.9e12).  128^3 x 8,192 atoms: 4.2 ms = 4.07 Tpair/s, the MUFU
+// unit 89 % busy, against 4.85 ms for a form with the atoms in pairs, eight FP32 operations a pair and
+// whole rows per thread; 61 x 57 x 50 x 777 atoms: 56 us for the call against 174.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,7 +29,21 @@
 namespace coul {
 
 constexpr int kAdjThreads = 128;
-constexpr int kAdjSegment = 256;
+
+// Shapes of the kernel by the grid columns X a thread holds in registers: rows per staged block,
+// chains of the block's FP32 charge sum (64 and 32 terms a lane: with 128 the charge gradient is less
+// exact than one row of 64 at a time) and resident CTAs per SM.  32 columns share a row's dy^2 + dz^2,
+// its sums and its loads of G among twice as many pairs: 4.07 Tpair/s on 128^3 x 8,192 against 3.93
+// with 16, which stay for row lengths that 32 would pad (16 warps of 124 registers against 20 of 92;
+// 8 columns: 3.64, two atoms a thread with 8 columns: 3.63).
+template <int X>
+struct AdjShape {
+    static constexpr int kRows = 256 / X;
+    static constexpr int kChains = X == 32 ? 2 : 4;
+    static constexpr int kBlocksPerSm = X == 32 ? 4 : 5;
+};
+constexpr int kAdjFoldRows = 64;   // terms of a column sum before it goes into FP64
+constexpr int kAdjReduceWarps = 8;
 
 struct AdjParams {
     const float4* atoms;
@@ -39,146 +56,164 @@ struct AdjParams {
     int chunks;
 };
 
-// Six CTAs per SM (at most 80 registers per thread, 24 warps): the pair loop's FMA and XU work is
-// balanced 8:1, so both pipes are busy at once and only more warps hide their dependency latency
-// (measured at 128^3 x 8,192 atoms: 4.87 ms with six CTAs and the point loop unrolled 4 times,
-// 5.11 ms with the 96-register, four-CTA form).
-template <int A>
-__global__ void __launch_bounds__(kAdjThreads, 6) adjoint_kernel(const AdjParams p)
+template <int X>
+__global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoint_kernel(const AdjParams p)
 {
-    __shared__ float4 s_pt[kAdjSegment];
+    constexpr int kRows = AdjShape<X>::kRows;
+    constexpr int kChains = AdjShape<X>::kChains;
+    constexpr int M = X / 2;                              // lane pairs of columns
+    constexpr int kPerThread = kRows * X / kAdjThreads;   // staged values per thread
+    static_assert(kRows * X % kAdjThreads == 0 && X % 4 == 0 && kRows <= kAdjThreads, "block shape");
+    // two buffers: a block is staged while slower warps still read the one before, one barrier a block
+    __shared__ __align__(16) float s_g[2][kRows * X];
+    __shared__ float2 s_row[2][kRows];  // the rows' (y, z)
     const int tid = threadIdx.x;
-    const int64_t tile_base = static_cast<int64_t>(blockIdx.x) * kAdjThreads * A;
-    float ax[A], ay[A], az[A];
-#pragma unroll
-    for (int k = 0; k < A; ++k) {
-        const int64_t j = tile_base + tid + static_cast<int64_t>(k) * kAdjThreads;
-        if (j < p.n_atoms) {
-            const float4 a = p.atoms[j];
-            ax[k] = a.x;
-            ay[k] = a.y;
-            az[k] = a.z;
-        } else {
-            ax[k] = ay[k] = az[k] = kPadCoord;  // far away; the result is never written
-        }
-    }
-    // FP64 per-atom accumulators, touched once per row: kept in shared memory (component-major, so
-    // a warp's accesses fall on consecutive words) rather than in 2 * 4 * A registers per thread,
-    // which lets more warps share an SM to hide the pair loop's dependency latency
-    __shared__ double s_acc[A * 4][kAdjThreads];
-#pragma unroll
-    for (int c = 0; c < A * 4; ++c)
-        s_acc[c][tid] = 0.0;
-
+    const int64_t j = static_cast<int64_t>(blockIdx.x) * kAdjThreads + tid;
+    // a thread past the last atom evaluates one far away and writes nothing
+    const float4 a = j < p.n_atoms ? p.atoms[j] : make_float4(kPadCoord, kPadCoord, kPadCoord, 0.0f);
     const int64_t rows = static_cast<int64_t>(p.ny) * p.nz;
     const int64_t r_begin = static_cast<int64_t>(blockIdx.y) * p.rows_per_chunk;
     const int64_t r_end = r_begin + p.rows_per_chunk < rows ? r_begin + p.rows_per_chunk : rows;
-    // Atoms in lane pairs (k = 2m, 2m + 1): the per-pair FP32 work runs as packed FFMA2 / FMUL2 /
-    // FADD2 instructions, two atoms per instruction, halving the issue slots the FMA pipe needs.
-    constexpr int P = A / 2;
-    static_assert(A % 2 == 0, "atoms per thread come in lane pairs");
-    float2 nax[P];
-#pragma unroll
-    for (int m = 0; m < P; ++m)
-        nax[m] = make_float2(-ax[2 * m], -ax[2 * m + 1]);
+    double tq = 0.0, tx = 0.0, ty = 0.0, tz = 0.0;
 
-    for (int64_t row = r_begin; row < r_end; ++row) {
-        const int y = static_cast<int>(row % p.ny);
-        const int z = static_cast<int>(row / p.ny);
-        const float gy = fmaf(static_cast<float>(y), p.h, p.oy);
-        const float gz = fmaf(static_cast<float>(z), p.h, p.oz);
-        float2 dyz2[P], sq[P], sx[P], s3[P];
+    // the next block's values travel through registers while the current one is evaluated
+    float next[kPerThread];
+    auto fetch = [&](int64_t row0, int x0) {
 #pragma unroll
-        for (int m = 0; m < P; ++m) {
-            const float dy0 = gy - ay[2 * m], dy1 = gy - ay[2 * m + 1];
-            const float dz0 = gz - az[2 * m], dz1 = gz - az[2 * m + 1];
-            dyz2[m] = make_float2(fmaf(dy0, dy0, dz0 * dz0), fmaf(dy1, dy1, dz1 * dz1));
-            sq[m] = make_float2(0.0f, 0.0f);
-            sx[m] = make_float2(0.0f, 0.0f);
-            s3[m] = make_float2(0.0f, 0.0f);
+        for (int i = 0; i < kPerThread; ++i) {
+            const int e = tid + i * kAdjThreads;
+            const int64_t row = row0 + e / X;
+            const int x = x0 + e % X;
+            next[i] = row < r_end && x < p.nx ? p.grad_map[row * p.nx + x] : 0.0f;
         }
-        const float* grow = p.grad_map + row * static_cast<int64_t>(p.nx);
-        for (int x0 = 0; x0 < p.nx; x0 += kAdjSegment) {
-            const int len = p.nx - x0 < kAdjSegment ? p.nx - x0 : kAdjSegment;
-            __syncthreads();
-            for (int i = tid; i < len; i += kAdjThreads) {
-                const float g = grow[x0 + i];
-                const float x = fmaf(static_cast<float>(x0 + i), p.h, p.ox);
-                s_pt[i] = make_float4(g, g, x, x);
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int i = 0; i < len; ++i) {
-                const float4 pt = s_pt[i];
-                const float2 g = make_float2(pt.x, pt.y);
-                const float2 gx = make_float2(pt.z, pt.w);
+    };
+    fetch(r_begin, 0);
+    int buf = 0;
+    for (int x0 = 0; x0 < p.nx; x0 += X) {
+        float2 dx[M], s3x[M];
 #pragma unroll
-                for (int m = 0; m < P; ++m) {
-                    const float2 dx = __fadd2_rn(gx, nax[m]);
-                    const float2 r2 = __ffma2_rn(dx, dx, dyz2[m]);
-                    const float2 inv = make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
-                    const float2 t = __fmul2_rn(g, inv);
-                    sq[m] = __fadd2_rn(sq[m], t);
-                    const float2 t3 = __fmul2_rn(t, __fmul2_rn(inv, inv));
-                    sx[m] = __ffma2_rn(t3, dx, sx[m]);
-                    s3[m] = __fadd2_rn(s3[m], t3);
-                }
-            }
-        }
-        // dy and dz recomputed here (same values as above) rather than held through the pair loop
-#pragma unroll
-        for (int m = 0; m < P; ++m) {
+        for (int m = 0; m < M; ++m) {
+            float d[2];
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
-                const int k = 2 * m + l;
-                const float vq = l ? sq[m].y : sq[m].x;
-                const float vx = l ? sx[m].y : sx[m].x;
-                const float v3 = l ? s3[m].y : s3[m].x;
-                const float dy = gy - ay[k];
-                const float dz = gz - az[k];
-                s_acc[4 * k + 0][tid] += static_cast<double>(vq);
-                s_acc[4 * k + 1][tid] += static_cast<double>(vx);
-                s_acc[4 * k + 2][tid] += static_cast<double>(dy) * static_cast<double>(v3);
-                s_acc[4 * k + 3][tid] += static_cast<double>(dz) * static_cast<double>(v3);
+                const int x = x0 + 2 * m + l;
+                // a column past the row's end lies far away (its staged G is zero)
+                d[l] = (x < p.nx ? fmaf(static_cast<float>(x), p.h, p.ox) : kPadCoord) - a.x;
+            }
+            dx[m] = make_float2(d[0], d[1]);
+            s3x[m] = make_float2(0.0f, 0.0f);
+        }
+        // the column sums into FP64: at the end of the rows, and every kAdjFoldRows rows
+        auto fold_x = [&]() {
+            float2 sx = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                sx = __ffma2_rn(dx[m], s3x[m], sx);
+                s3x[m] = make_float2(0.0f, 0.0f);
+            }
+            tx += static_cast<double>(sx.x + sx.y);
+        };
+        int unfolded = 0;
+        for (int64_t row0 = r_begin; row0 < r_end; row0 += kRows) {
+            const int count = static_cast<int>(r_end - row0 < kRows ? r_end - row0 : kRows);
+            buf ^= 1;
+#pragma unroll
+            for (int i = 0; i < kPerThread; ++i)
+                s_g[buf][tid + i * kAdjThreads] = next[i];
+            if (tid < count) {
+                const int64_t row = row0 + tid;
+                s_row[buf][tid] = make_float2(fmaf(static_cast<float>(static_cast<int>(row % p.ny)), p.h, p.oy),
+                                         fmaf(static_cast<float>(static_cast<int>(row / p.ny)), p.h, p.oz));
+            }
+            __syncthreads();
+            if (row0 + kRows < r_end)
+                fetch(row0 + kRows, x0);
+            else
+                fetch(r_begin, x0 + X);
+            float2 sq[kChains];
+#pragma unroll
+            for (int i = 0; i < kChains; ++i)
+                sq[i] = make_float2(0.0f, 0.0f);
+            float sy = 0.0f, sz = 0.0f;
+            for (int r = 0; r < count; ++r) {
+                const float2 yz = s_row[buf][r];
+                const float dy = yz.x - a.y;
+                const float dz = yz.y - a.z;
+                const float2 dyz2 = splat(fmaf(dy, dy, dz * dz));
+                const float4* g4 = reinterpret_cast<const float4*>(s_g[buf] + r * X);
+                float2 s3r = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const float4 gq = g4[m / 2];
+                    const float2 g = m & 1 ? make_float2(gq.z, gq.w) : make_float2(gq.x, gq.y);
+                    const float2 r2 = __ffma2_rn(dx[m], dx[m], dyz2);
+                    const float2 inv = rsqrt_mufu_x2(r2);
+                    const float2 inv3 = __fmul2_rn(__fmul2_rn(inv, inv), inv);
+                    sq[m % kChains] = __ffma2_rn(g, inv, sq[m % kChains]);
+                    s3x[m] = __ffma2_rn(g, inv3, s3x[m]);
+                    s3r = m == 0 ? __fmul2_rn(g, inv3) : __ffma2_rn(g, inv3, s3r);
+                }
+                const float v = s3r.x + s3r.y;
+                sy = fmaf(dy, v, sy);
+                sz = fmaf(dz, v, sz);
+            }
+            float2 q = sq[0];
+#pragma unroll
+            for (int i = 1; i < kChains; ++i)
+                q = __fadd2_rn(q, sq[i]);
+            tq += static_cast<double>(q.x + q.y);
+            ty += static_cast<double>(sy);
+            tz += static_cast<double>(sz);
+            unfolded += kRows;
+            if (unfolded == kAdjFoldRows) {
+                fold_x();
+                unfolded = 0;
             }
         }
+        fold_x();
     }
-
-#pragma unroll
-    for (int k = 0; k < A; ++k) {
-        const int64_t j = tile_base + tid + static_cast<int64_t>(k) * kAdjThreads;
-        if (j < p.n_atoms) {
-            double* dst = p.partial + (static_cast<int64_t>(blockIdx.y) * p.n_atoms + j) * 4;
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                dst[c] = s_acc[4 * k + c][tid];
-        }
+    if (j < p.n_atoms) {
+        double2* dst = reinterpret_cast<double2*>(p.partial + (static_cast<int64_t>(blockIdx.y) * p.n_atoms + j) * 4);
+        dst[0] = make_double2(tq, tx);
+        dst[1] = make_double2(ty, tz);
     }
 }
 
-// dq_j = sum over chunks of the partial sum; dr_j = q_j * (sum of the three position partials);
-// chunks added in index order.
-__global__ void adjoint_reduce_kernel(const float4* __restrict__ atoms, const double* __restrict__ partial, int64_t n,
-                                      int chunks, float* __restrict__ grad_q, float* __restrict__ grad_xyz)
+// dq_j = sum over chunks of the partial sum; dr_j = q_j * (sum of the three position partials).  A
+// warp's lanes are the 4 components of 8 consecutive atoms (256 contiguous bytes of each chunk); warp
+// w of the block adds the chunks w, w + 8, ... in order, then the warps' sums are added in warp order.
+// One thread per atom over all chunks took as long as the gradient itself for a small molecule.
+__global__ void __launch_bounds__(32 * kAdjReduceWarps) adjoint_reduce_kernel(
+    const float4* __restrict__ atoms, const double* __restrict__ partial, int64_t n, int chunks,
+    float* __restrict__ grad_q, float* __restrict__ grad_xyz, float4* __restrict__ grad)
 {
-    const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j >= n)
+    __shared__ double s_sum[kAdjReduceWarps][32];
+    const int lane = threadIdx.x % 32;
+    const int warp = threadIdx.x / 32;
+    const int64_t e = static_cast<int64_t>(blockIdx.x) * 32 + lane;  // element (atom, component)
+    double s = 0.0;
+    if (e < 4 * n) {
+#pragma unroll 8
+        for (int c = warp; c < chunks; c += kAdjReduceWarps)
+            s += partial[static_cast<int64_t>(c) * 4 * n + e];
+    }
+    s_sum[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0 || e >= 4 * n)
         return;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int c = 0; c < chunks; ++c) {
-        const double* src = partial + (static_cast<int64_t>(c) * n + j) * 4;
+    s = s_sum[0][lane];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            s[k] += src[k];
-    }
-    const double q = static_cast<double>(atoms[j].w);
-    if (grad_q)
-        grad_q[j] = static_cast<float>(s[0]);
-    if (grad_xyz) {
-        grad_xyz[3 * j + 0] = static_cast<float>(q * s[1]);
-        grad_xyz[3 * j + 1] = static_cast<float>(q * s[2]);
-        grad_xyz[3 * j + 2] = static_cast<float>(q * s[3]);
-    }
+    for (int w = 1; w < kAdjReduceWarps; ++w)
+        s += s_sum[w][lane];
+    const int64_t j = e / 4;
+    const int k = static_cast<int>(e % 4);
+    const float v = static_cast<float>(k == 0 ? s : static_cast<double>(atoms[j].w) * s);
+    if (grad)
+        reinterpret_cast<float*>(grad)[4 * j + (k == 0 ? 3 : k - 1)] = v;  // (dx, dy, dz, dq)
+    if (k == 0 && grad_q)
+        grad_q[j] = v;
+    if (k != 0 && grad_xyz)
+        grad_xyz[3 * j + k - 1] = v;
 }
 
 struct AdjointWorkspace {
@@ -190,8 +225,15 @@ struct AdjointWorkspace {
 
 using namespace coul;
 
-extern "C" COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
-                                        const float* d_grad_map, float* d_grad_q, float* d_grad_xyz)
+template <int X>
+static void launch_adjoint(const AdjParams& p, int64_t tiles, cudaStream_t stream)
+{
+    adjoint_kernel<X><<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(p.chunks)), kAdjThreads, 0, stream>>>(p);
+}
+
+// The call of both entry points: any of the three outputs may be NULL.
+static int adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid, const float* d_grad_map,
+                      float* d_grad_q, float* d_grad_xyz, float* d_grad)
 {
     if (ctx == nullptr)
         return set_error(COUL_ERR_INVALID_ARGUMENT, "ctx is NULL");
@@ -199,20 +241,29 @@ extern "C" COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int
     if (rc)
         return rc;
     if (n_atoms < 0 || d_grad_map == nullptr || (n_atoms > 0 && (d_atoms == nullptr || !aligned16(d_atoms))) ||
-        (d_grad_q == nullptr && d_grad_xyz == nullptr))
+        (d_grad_q == nullptr && d_grad_xyz == nullptr && d_grad == nullptr))
         return set_error(COUL_ERR_INVALID_ARGUMENT, "bad atoms, gradient map or outputs");
     if (n_atoms == 0)
         return COUL_OK;
     if ((rc = ctx_activate(ctx)))
         return rc;
 
-    constexpr int A = 4;
-    const int64_t tiles = (n_atoms + kAdjThreads * A - 1) / (kAdjThreads * A);
+    const int64_t tiles = (n_atoms + kAdjThreads - 1) / kAdjThreads;
     const int64_t rows = static_cast<int64_t>(grid->ny) * grid->nz;
-    // enough (tile, chunk) CTAs for ~4 waves of 6 per SM, without chunks shorter than 8 rows
-    const int64_t target = static_cast<int64_t>(ctx->sm_count) * 24;
-    int64_t chunks = std::max<int64_t>(1, std::min<int64_t>((target + tiles - 1) / tiles, (rows + 7) / 8));
-    chunks = std::min<int64_t>(chunks, 65535);
+    // 32 columns a thread unless they pad the rows by more than the 4 % they gain over 16
+    const auto padded = [&](int64_t x) { return (grid->nx + x - 1) / x * x; };
+    const bool wide = padded(32) * 100 <= padded(16) * 104;
+    // Equal (tile, chunk) CTAs in whole waves of the resident ones, rounded down so that no wave is
+    // nearly empty: as many waves (at most 8; the SMs' warps drift apart within one) as leave a chunk
+    // 32 rows, else one wave.
+    const int64_t slots = static_cast<int64_t>(ctx->sm_count) * (wide ? AdjShape<32>::kBlocksPerSm : AdjShape<16>::kBlocksPerSm);
+    int64_t chunks = 1;
+    for (int64_t waves = 8; waves >= 1; --waves) {
+        chunks = std::max<int64_t>(1, waves * slots / tiles);
+        if (rows / chunks >= 32)
+            break;
+    }
+    chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, std::min<int64_t>((rows + 3) / 4, 65535)));
     const int64_t rows_per_chunk = (rows + chunks - 1) / chunks;
     chunks = (rows + rows_per_chunk - 1) / rows_per_chunk;
     if (tiles > 2147483647LL)
@@ -260,12 +311,31 @@ extern "C" COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int
     p.chunks = static_cast<int>(chunks);
     if ((rc = ctx_begin_timing(ctx)))
         return rc;
-    adjoint_kernel<A><<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(chunks)), kAdjThreads, 0, ctx->stream>>>(p);
+    if (wide)
+        launch_adjoint<32>(p, tiles, ctx->stream);
+    else
+        launch_adjoint<16>(p, tiles, ctx->stream);
     if ((e = cudaGetLastError()) != cudaSuccess)
         return cuda_error(e, "adjoint launch");
-    adjoint_reduce_kernel<<<static_cast<unsigned>((n_atoms + 255) / 256), 256, 0, ctx->stream>>>(
-        p.atoms, ws->partial, n_atoms, p.chunks, d_grad_q, d_grad_xyz);
+    adjoint_reduce_kernel<<<static_cast<unsigned>((n_atoms + 7) / 8), 32 * kAdjReduceWarps, 0, ctx->stream>>>(
+        p.atoms, ws->partial, n_atoms, p.chunks, d_grad_q, d_grad_xyz, reinterpret_cast<float4*>(d_grad));
     if ((e = cudaGetLastError()) != cudaSuccess)
         return cuda_error(e, "adjoint reduction launch");
     return ctx_end_timing(ctx);
 }
+
+extern "C" {
+
+COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
+                             const float* d_grad_map, float* d_grad_q, float* d_grad_xyz)
+{
+    return adjoint_3d(ctx, d_atoms, n_atoms, grid, d_grad_map, d_grad_q, d_grad_xyz, nullptr);
+}
+
+COUL_API int coul_adjoint_3d_packed(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
+                                    const float* d_grad_map, float* d_grad)
+{
+    return adjoint_3d(ctx, d_atoms, n_atoms, grid, d_grad_map, nullptr, nullptr, d_grad);
+}
+
+}  // extern "C"

@@ -189,3 +189,25 @@ def test_adam_charge_fitting_full_size(ctx):
     q_err = np.abs(q.detach().cpu().numpy() - q_target).mean()
     assert losses[-1] < 0.5 * losses[0], losses[::10]
     assert q_err <= q_err0, (q_err, q_err0)
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 400])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (16, 3, 5), (31, 9, 4), (32, 8, 9), (33, 40, 3), (49, 2, 37), (65, 130, 1)])
+def test_adjoint_block_edges(ctx, dims, n):
+    """Row lengths around the kernel's column blocks (16 and 32), row counts around its staged blocks
+    and chunks, atom counts around a CTA's 128, against the FP64 gradient.  L = 0.5 sum V^2 with T = 0
+    and w = 1, so G = V: an FP32 pair chain is good to about 4e-7 of its own magnitude and the sums
+    here cancel by less than a factor of ten in the largest component; 1e-5 of it."""
+    import torch
+    rng = np.random.default_rng(1000 * n + dims[0])
+    atoms = np.empty((n, 4), dtype=np.float32)
+    atoms[:, :3] = rng.uniform(-4.0, 0.5 * max(dims) + 4.0, (n, 3))
+    atoms[:, 3] = rng.uniform(0.2, 1.0, n)
+    h, origin = 0.5, (0.25, -0.5, 1.0)
+    v = oracle.grid3d(atoms, h, dims, origin).astype(np.float32)
+    zero, one = np.zeros_like(v), np.ones_like(v)
+    _, dq, dr = oracle.adjoint3d(atoms, h, dims, zero, one, origin=origin)
+    got = ktt_b200.adjoint_3d(ctx, torch.from_numpy(atoms).cuda(), dims, h, torch.from_numpy(v).cuda(), origin)
+    got = got.cpu().numpy().astype(np.float64)
+    assert _rel(got[:, 3], dq) <= 1e-5
+    assert _rel(got[:, :3], dr) <= 1e-5
