@@ -51,6 +51,7 @@ struct FwdParams {
     float h, ox, oy, oz;
     float* out;
     int accumulate;
+    int columns;  // 3D, one CTA per tile: columns of x points per row of linear x-y tiles, 0 for the block's rectangles
     int* status;
 };
 

@@ -319,3 +319,28 @@ def test_fp64_merge_shared_sums_equal_register_sums(ctx, tune):
     assert torch.equal(reg, shr)
     ref = oracle.grid3d(a, h, dims, origin)
     assert errors.report(shr.cpu().numpy(), ref)["rel_norm"] <= 1e-5
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 300, 1), (131, 3, 9), (129, 7, 17), (257, 2, 8), (96, 33, 5)])
+@pytest.mark.parametrize("tune", [
+    ktt_b200.Tune(block_x=64, block_y=1, z_iterations=8, x_points=2, unroll=2, rsqrt_soft=2),
+    ktt_b200.Tune(block_x=64, block_y=1, z_iterations=8, x_points=4, precision=ktt_b200.PREC_FP64_PAIRS),
+    ktt_b200.Tune(block_x=7, block_y=3, z_iterations=4, x_points=1, atom_source=ktt_b200.ATOMS_CONSTANT),
+    ktt_b200.Tune(block_x=16, block_y=8, z_iterations=16, x_points=2, rsqrt_soft=12,
+                  precision=ktt_b200.PREC_FP64_MERGE_SHARED),
+])
+def test_linear_and_rectangular_tiles(ctx, dims, tune):
+    """Planes that the block's rectangles pad by a little, a lot and not at all (the launch picks linear
+    x-y tiles or the rectangles): within the norm tolerance of the oracle, and the points of a
+    row-by-row launch (block of one row, no linear tile can be fewer) bit for bit."""
+    import torch
+    rng = np.random.default_rng(sum(dims))
+    a = np.empty((77, 4), dtype=np.float32)
+    a[:, :3] = rng.uniform(0.0, 0.5 * max(dims), (77, 3))
+    a[:, 3] = rng.uniform(-1.0, 1.0, 77)
+    h, origin = 0.5, (-1.0, 0.5, 2.0)
+    out = torch.full((dims[2], dims[1], dims[0]), float("nan"), device="cuda")
+    ctx.forward_3d(_t(a), dims, h, origin, tune=tune, out=out)
+    assert errors.report(_np(out), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
+    row = ktt_b200.Tune(**dict(tune.as_dict(), block_x=1, block_y=1))
+    assert torch.equal(out, ctx.forward_3d(_t(a), dims, h, origin, tune=row))
