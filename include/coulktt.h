@@ -272,12 +272,25 @@ COUL_API int coul_pack_atoms(coul_ctx* ctx, const float* d_x, const float* d_y, 
 COUL_API int coul_slice_atoms(coul_ctx* ctx, const float* d_xyzq, int64_t n_atoms, float z_slice,
                               float* d_xy_dz2_q);
 /*
+ * The 3D map, or its slab [z_begin, z_end), and the 2D slice without a configuration: kernels that
+ * suit every grid size (csrc/coul_plain.cu), FP32 pairs, sums at least as exact as those of
+ * coul_tune_default().  Slabs put together equal the whole map bit for bit, whatever their
+ * boundaries.  No counterpart in the reference, whose tuner picks a configuration for every launch.
+ */
+COUL_API int coul_forward_3d_plain(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
+                                   int z_begin, int z_end, int accumulate, float* d_out);
+COUL_API int coul_forward_2d_plain(coul_ctx* ctx, const float* d_atoms_xy_dz2_q, int64_t n_atoms, float spacing, int nx,
+                                   int ny, int accumulate, float* d_out);
+/*
  * Host-buffer convenience call: uploads h_atoms, computes the 3D map (out = V)
  * and downloads it into h_out, then waits.  Device buffers are cached in the
  * context and grown on demand.
  */
 COUL_API int coul_forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
                                   const coul_tune* tune, float* h_out);
+/* The same without a configuration (coul_forward_3d_plain). */
+COUL_API int coul_forward_3d_host_plain(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
+                                        float* h_out);
 
 /* ---- adjoint: gradient of a loss on the map ----------------------------------------- */
 /*

@@ -134,6 +134,8 @@ def load_library():
         "coul_variant_count": [],
         "coul_variant_get": [ci, T, ctypes.POINTER(ci), ctypes.POINTER(ci)],
         "coul_forward_3d": [vp, vp, i64, G, T, ci, vp],
+        "coul_forward_3d_plain": [vp, vp, i64, G, ci, ci, ci, vp],
+        "coul_forward_2d_plain": [vp, vp, i64, cf, ci, ci, ci, vp],
         "coul_forward_3d_slab": [vp, vp, i64, G, ci, ci, T, ci, vp],
         "coul_forward_3d_soa": [vp, vp, vp, vp, vp, i64, G, T, ci, vp],
         "coul_forward_3d_reference": [vp, vp, i64, G, ci, vp],
@@ -141,6 +143,7 @@ def load_library():
         "coul_forward_2d": [vp, vp, i64, cf, ci, ci, T, ci, vp],
         "coul_slice_atoms": [vp, vp, i64, cf, vp],
         "coul_forward_3d_host": [vp, vp, i64, G, T, vp],
+        "coul_forward_3d_host_plain": [vp, vp, i64, G, vp],
         "coul_probe_bounded_wait": [vp, ci, ctypes.c_uint64],
         "coul_measure_pipe_rates": [vp, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)],
         "coul_measure_pipe_rates_ex": [vp, ctypes.POINTER(_PipeRates)],
@@ -294,13 +297,18 @@ class CoulombContext:
     # -- forward ------------------------------------------------------------------------------
     def forward_3d(self, atoms, dims, spacing, origin=None, tune: Tune | None = None, out=None,
                    accumulate: bool = False):
-        """Map of shape (nz, ny, nx) for dims = (nx, ny, nz)."""
+        """Map of shape (nz, ny, nx) for dims = (nx, ny, nz).  Without a tune the library's plain kernels
+        choose their own shape for the grid (coul_forward_3d_plain)."""
         self._check_atoms(atoms)
         nx, ny, nz = (int(d) for d in dims)
         out = self._out(out, (nz, ny, nx), atoms.device)
         self._bind_stream()
         g = _grid(dims, spacing, origin)
-        t = (tune or Tune()).c()
+        if tune is None:
+            _check(self._lib.coul_forward_3d_plain(self._ctx, _ptr(atoms), atoms.shape[0], ctypes.byref(g), 0, nz,
+                                                   1 if accumulate else 0, _ptr(out)))
+            return out
+        t = tune.c()
         _check(self._lib.coul_forward_3d(self._ctx, _ptr(atoms), atoms.shape[0], ctypes.byref(g), ctypes.byref(t),
                                          1 if accumulate else 0, _ptr(out)))
         return out
@@ -308,14 +316,18 @@ class CoulombContext:
     def forward_3d_slab(self, atoms, dims, spacing, z_begin: int, z_end: int, origin=None,
                         tune: Tune | None = None, out=None, accumulate: bool = False):
         """Slab z in [z_begin, z_end) of the map of dims = (nx, ny, nz): shape (z_end - z_begin, ny, nx),
-        the full grid's point coordinates (slabs starting at multiples of tune.z_iterations put together
-        equal forward_3d bit for bit)."""
+        the full grid's point coordinates (slabs starting at multiples of tune.z_iterations, or any
+        slabs without a tune, put together equal forward_3d bit for bit)."""
         self._check_atoms(atoms)
         nx, ny, nz = (int(d) for d in dims)
         out = self._out(out, (int(z_end) - int(z_begin), ny, nx), atoms.device)
         self._bind_stream()
         g = _grid(dims, spacing, origin)
-        t = (tune or Tune()).c()
+        if tune is None:
+            _check(self._lib.coul_forward_3d_plain(self._ctx, _ptr(atoms), atoms.shape[0], ctypes.byref(g),
+                                                   int(z_begin), int(z_end), 1 if accumulate else 0, _ptr(out)))
+            return out
+        t = tune.c()
         _check(self._lib.coul_forward_3d_slab(self._ctx, _ptr(atoms), atoms.shape[0], ctypes.byref(g), int(z_begin),
                                               int(z_end), ctypes.byref(t), 1 if accumulate else 0, _ptr(out)))
         return out
@@ -363,7 +375,11 @@ class CoulombContext:
         self._check_atoms(atoms_xy_dz2_q)
         out = self._out(out, (int(ny), int(nx)), atoms_xy_dz2_q.device)
         self._bind_stream()
-        t = (tune or Tune(block_x=32, block_y=4, z_iterations=4, x_points=4)).c()
+        if tune is None:
+            _check(self._lib.coul_forward_2d_plain(self._ctx, _ptr(atoms_xy_dz2_q), atoms_xy_dz2_q.shape[0],
+                                                   float(spacing), int(nx), int(ny), 1 if accumulate else 0, _ptr(out)))
+            return out
+        t = tune.c()
         _check(self._lib.coul_forward_2d(self._ctx, _ptr(atoms_xy_dz2_q), atoms_xy_dz2_q.shape[0], float(spacing),
                                          int(nx), int(ny), ctypes.byref(t), 1 if accumulate else 0, _ptr(out)))
         return out
@@ -384,7 +400,11 @@ class CoulombContext:
         out = np.empty((nz, ny, nx), dtype=np.float32) if out_np is None else out_np
         assert out.flags.c_contiguous and out.dtype == np.float32 and out.size == nx * ny * nz
         g = _grid(dims, spacing, origin)
-        t = (tune or Tune()).c()
+        if tune is None:
+            _check(self._lib.coul_forward_3d_host_plain(self._ctx, a.ctypes.data, a.shape[0], ctypes.byref(g),
+                                                        out.ctypes.data))
+            return out
+        t = tune.c()
         _check(self._lib.coul_forward_3d_host(self._ctx, a.ctypes.data, a.shape[0], ctypes.byref(g), ctypes.byref(t),
                                               out.ctypes.data))
         return out

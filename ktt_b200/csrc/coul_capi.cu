@@ -1010,15 +1010,16 @@ COUL_API int coul_probe_bounded_wait(coul_ctx* ctx, int arrive, uint64_t budget_
     return coul_synchronize(ctx);
 }
 
-COUL_API int coul_forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
-                                  const coul_tune* tune, float* h_out)
+// tune NULL: the plain map
+static int forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
+                           const coul_tune* tune, float* h_out)
 {
     if (ctx == nullptr)
         return set_error(COUL_ERR_INVALID_ARGUMENT, "ctx is NULL");
     int rc = validate_grid(grid);
     if (rc)
         return rc;
-    if ((rc = validate_tune(tune, kModeGrid3d, 0, nullptr)))
+    if (tune && (rc = validate_tune(tune, kModeGrid3d, 0, nullptr)))
         return rc;
     if (n_atoms < 0 || h_out == nullptr || (n_atoms > 0 && h_atoms == nullptr))
         return set_error(COUL_ERR_INVALID_ARGUMENT, "bad host buffers");
@@ -1048,11 +1049,29 @@ COUL_API int coul_forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n
     if (abytes > 0 &&
         (e = cudaMemcpyAsync(ctx->d_atoms_cache, h_atoms, abytes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_error(e, "atom upload");
-    if ((rc = coul_forward_3d(ctx, ctx->d_atoms_cache, n_atoms, grid, tune, 0, ctx->d_out_cache)))
+    rc = tune ? coul_forward_3d(ctx, ctx->d_atoms_cache, n_atoms, grid, tune, 0, ctx->d_out_cache)
+              : coul_forward_3d_plain(ctx, ctx->d_atoms_cache, n_atoms, grid, 0, grid->nz, 0, ctx->d_out_cache);
+    if (rc)
         return rc;
     if ((e = cudaMemcpyAsync(h_out, ctx->d_out_cache, obytes, cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess)
         return cuda_error(e, "map download");
     return coul_synchronize(ctx);
+}
+
+COUL_API int coul_forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
+                                  const coul_tune* tune, float* h_out)
+{
+    if (ctx != nullptr && tune == nullptr) {
+        const int rc = validate_grid(grid);
+        return rc ? rc : validate_tune(nullptr, kModeGrid3d, 0, nullptr);
+    }
+    return forward_3d_host(ctx, h_atoms, n_atoms, grid, tune, h_out);
+}
+
+COUL_API int coul_forward_3d_host_plain(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
+                                        float* h_out)
+{
+    return forward_3d_host(ctx, h_atoms, n_atoms, grid, nullptr, h_out);
 }
 
 }  // extern "C"
