@@ -82,7 +82,8 @@ enum {
 enum {
     COUL_PREC_FP32 = 0,        /* one FP32 accumulator per point (KTT's kernel) */
     COUL_PREC_COMPENSATED = 1, /* FP32 partial per 64-atom sub-tile, merged by two-sum into (sum, error) */
-    COUL_PREC_FP64_MERGE = 2,  /* FP32 partial per 64-atom sub-tile, merged into an FP64 accumulator */
+    COUL_PREC_FP64_MERGE = 2,  /* FP32 partial per 64-atom sub-tile (48 with 2 x 16 points a thread), merged
+                                  into an FP64 accumulator */
     COUL_PREC_FP64_PAIRS = 3,  /* every pair in FP64: exact differences, FP64 r^2, MUFU rsqrt estimate
                                   refined by one FP64 Newton step (about 2^-40), FP64 accumulation; the
                                   map's error is then its FP32 store.  3D maps, rsqrt_soft 0 only */
@@ -113,8 +114,9 @@ typedef struct coul_tune {
                          the atom-split form also the warps of a block) take turns in 8 / n phases
                          and pair p in phase g is on the FMA pipe when g * n + p < rsqrt_soft.  Either
                          way the share is rsqrt_soft / 8.
-                         10 + k (k = 0..7): successive patterns alternate between k and k + 1 eighths,
-                         a share of (2k + 1) / 16 */
+                         10 + k (k = 0..7): a share of (2k + 1) / 16: with n >= 16 that many of every
+                         16 pairs, spread evenly; with fewer, successive patterns alternate between k
+                         and k + 1 eighths */
     int atom_split;   /* 0 or 1: one CTA per point tile; 2 or more: the atoms are split into that
                          many chunks per point tile, the partial sums of a tile added in chunk order
                          (for slices and small maps with too few tiles to fill the GPU; FP32,

@@ -55,6 +55,8 @@ static const std::vector<BatchVariant>& batch_variants()
         // FP64 merge with the sums in shared memory (the pointwise-accurate form with fewer registers)
         batch_variant<8, 2, 1, kPrecFp64MergeShared, 2>(), batch_variant<8, 2, 2, kPrecFp64MergeShared, 2>(),
         batch_variant<16, 1, 1, kPrecFp64MergeShared, 2>(), batch_variant<4, 4, 1, kPrecFp64MergeShared, 2>(),
+        // record tiles (32 points a thread), 5/16 of the rsqrts on the FMA pipe
+        batch_variant<16, 2, 1, kPrecFp64MergeShared, kSoftAlternate + 2>(),
     };
     return v;
 }
@@ -214,9 +216,7 @@ COUL_API int coul_batch_create(coul_ctx* ctx, const coul_molecule* molecules, in
 
     cudaError_t e;
     int blocks_per_sm = 0;
-    b->smem = kStages * kTileAtoms * 16 + kStages * 8;
-    if (b->tune.precision == COUL_PREC_FP64_MERGE_SHARED)
-        b->smem += shared_sums_bytes(threads, b->tune.z_iterations * b->tune.x_points);
+    b->smem = tile_smem_bytes(threads, b->tune.z_iterations, b->tune.x_points, 0, b->tune.precision, kModeGrid3d);
     if (b->smem > 48u * 1024u &&
         (e = cudaFuncSetAttribute(b->variant->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(b->smem))) != cudaSuccess) {
@@ -328,7 +328,7 @@ COUL_API int coul_batch_run(coul_ctx* ctx, coul_batch* b, int mode, int accumula
             p.oz = m.grid.origin[2];
             p.out = m.d_out;
             p.accumulate = accumulate;
-            if ((rc = launch_forward(ctx, v, p, kModeGrid3d, &t)))
+            if ((rc = launch_forward(ctx, v, p, kModeGrid3d, &t, 0)))
                 return rc;
         }
         break;

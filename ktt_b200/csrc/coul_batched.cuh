@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) ba
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + kStages * kTileAtoms * 16);
     __shared__ long long s_item;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    ring_init(full, tid);
+    if constexpr (!record_tile(ZI, XP, kSrcShared, 0, PREC, kModeGrid3d))
+        ring_init(full, tid);
     uint32_t gstage = 0;
 
     for (;;) {

@@ -445,9 +445,46 @@ int queue_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const 
     return COUL_OK;
 }
 
+// The atom split of record tiles (record_split_kernel) on a map of nz planes: warps per tile, CTAs per
+// tile and planes per tile, from the whole grid and the atom count alone.
+static void record_split_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tune* t, int nz)
+{
+    const int zi = t->z_iterations;
+    const int columns = (L.p.nx + t->x_points - 1) / t->x_points;
+    const int64_t tiles_xy = (static_cast<int64_t>(columns) * L.p.ny + 31) / 32;
+    const auto tiles_at = [&](int depth) { return tiles_xy * ((nz + depth - 1) / depth); };
+    const int64_t tiles = tiles_at(zi);
+    const int64_t partials = (L.p.n_atoms + kRecordMerge - 1) / kRecordMerge;
+    // Warps per tile: more until the map has 54 of them an SM (16 are resident: three to four rounds), and
+    // beyond that while each keeps 13 partials.  us by warps per tile (1, 2, 4, 8) on B200: 128^3 x 500 atoms
+    // 233, 230, 212, 221; 64^3 x 500 90, 74, 45, 42; 224^3 x 300 608, 625, 661, 688; 224^3 x 5,000 9,798,
+    // 9,741, 9,710, 9,626.
+    int group = 1;
+    while (group < kRecordSplitWarps && (tiles * group < 54LL * ctx->sm_count || partials >= 26LL * group))
+        group *= 2;
+    if (group == 1)
+        return;  // fwd_kernel
+    // half the depth, then more CTAs a tile, while there are fewer CTAs than SMs
+    const int per_cta = kRecordSplitWarps / group;
+    const int depth = group == kRecordSplitWarps && tiles < ctx->sm_count ? zi / 2 : zi;
+    int ranks = 1;
+    while (group == kRecordSplitWarps && ranks < kMaxPortableSplit && tiles_at(depth) * ranks < ctx->sm_count &&
+           partials >= 2 * ranks * kRecordSplitWarps)
+        ranks *= 2;
+    if (tiles_xy * ranks > 2147483647LL || (nz + depth - 1) / depth > 65535)
+        return;
+    L.record_group = group;
+    L.record_ranks = ranks;
+    L.record_depth = depth;
+    L.p.columns = columns;
+    L.smem = record_split_smem_bytes(zi, t->x_points);
+    L.grid = dim3(static_cast<unsigned>((tiles_xy + per_cta - 1) / per_cta * ranks),
+                  static_cast<unsigned>((L.p.nz - L.p.z_base + depth - 1) / depth), 1);
+}
+
 // Launch one forward variant over a grid; shared by the 3D AoS/SoA and 2D entry points and by
 // the batched path's plain-launch baseline.
-int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t)
+int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz)
 {
     FwdLaunch L{};
     L.p = prm;
@@ -479,9 +516,12 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
             L.grid.y = static_cast<unsigned>(rows);
         }
     }
-    L.smem = (t->atom_source == COUL_ATOMS_SHARED_TMA) ? (kStages * kTileAtoms * 16 + kStages * 8) : 0;
-    if (t->precision == COUL_PREC_FP64_MERGE_SHARED)
-        L.smem += shared_sums_bytes(t->block_x * t->block_y, t->z_iterations * t->x_points);
+    L.smem = t->atom_source == COUL_ATOMS_SHARED_TMA
+                 ? tile_smem_bytes(t->block_x * t->block_y, t->z_iterations, t->x_points, v->key.soa, t->precision, mode)
+                 : 0;
+    if (nz > 0 && v->key.split == 0 && t->precision != COUL_PREC_FP32 &&
+        record_tile(t->z_iterations, t->x_points, t->atom_source, v->key.soa, t->precision, mode))
+        record_split_setup(ctx, L, t, nz);
     if (v->key.split == 1) {
         L.split = t->atom_split;
         L.smem = split_smem_bytes(t->block_x * t->block_y, t->z_iterations * t->x_points);
@@ -843,7 +883,7 @@ static int forward_3d_common(coul_ctx* ctx, const float* d_atoms, const float* d
     p.accumulate = accumulate ? 1 : 0;
     if ((rc = ctx_begin_timing(ctx)))
         return rc;
-    if ((rc = launch_forward(ctx, v, p, kModeGrid3d, tune)))
+    if ((rc = launch_forward(ctx, v, p, kModeGrid3d, tune, grid->nz)))
         return rc;
     return ctx_end_timing(ctx);
 }
@@ -952,7 +992,7 @@ COUL_API int coul_forward_2d(coul_ctx* ctx, const float* d_atoms, int64_t n_atom
     p.accumulate = accumulate ? 1 : 0;
     if ((rc = ctx_begin_timing(ctx)))
         return rc;
-    if ((rc = launch_forward(ctx, v, p, kModeSlice2d, tune)))
+    if ((rc = launch_forward(ctx, v, p, kModeSlice2d, tune, 0)))
         return rc;
     return ctx_end_timing(ctx);
 }

@@ -184,6 +184,13 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr)
     return v;
 }
 
+__device__ __forceinline__ double ld_cluster_f64(uint32_t addr)
+{
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 // MUFU reciprocal square root (approximate, flush-to-zero), the instruction KTT's kernels reach
 // through rsqrt()/half_rsqrt() under fast-math.
 __device__ __forceinline__ float rsqrt_mufu(float x)
@@ -260,13 +267,18 @@ __device__ __forceinline__ float2 rsqrt_fma_x2(float2 x)
 // slot s = (stage phase) * NP + p for NP < 8, s = p % 8 otherwise, and a slot takes the FMA pipe
 // when s < SOFT.  The share is SOFT / 8 at every tile size.  From kSoftAlternate on
 // (SOFT = kSoftAlternate + k) two such patterns alternate between k and k + 1 soft slots, a share
-// of (2k + 1) / 16.  soft_phases is the number of stage phases of one whole pattern.
+// of (2k + 1) / 16; with NP >= 16 that share fits into one pattern, and pair p is soft where
+// (p + 1) (2k + 1) / 16 passes a whole number: 2k + 1 of every 16 pairs, spread evenly, so that a run of
+// MUFU pairs and a run of FMA-pipe pairs never wait for one another (5/16 of 16 pairs in a bare pair
+// loop: 6.30 Tpair/s spread, 6.05 side by side).  soft_phases is the number of stage phases of one whole
+// pattern.
 constexpr int kSoftAlternate = 10;
 constexpr int soft_group(int np) { return np >= 8 ? 1 : 8 / np; }
 constexpr int soft_phases(int soft, int np)
 {
-    return soft == 0 ? 1 : (soft >= kSoftAlternate ? 2 : 1) * soft_group(np);
+    return soft == 0 || np >= 16 ? 1 : (soft >= kSoftAlternate ? 2 : 1) * soft_group(np);
 }
+constexpr bool spread_soft(int p, int sixteenths) { return (p + 1) * sixteenths / 16 != p * sixteenths / 16; }
 
 // Calls f(std::integral_constant<int, phase>) for a run-time phase in [0, P): the stage loop is
 // instantiated once per phase so that the soft/MUFU choice stays a compile-time one per pair.
@@ -286,6 +298,8 @@ __device__ __forceinline__ void with_phase(const int phase, F&& f)
 template <int SOFT, int NP, int PHASE>
 __device__ __forceinline__ constexpr bool pair_is_soft(int p)
 {
+    if constexpr (SOFT >= kSoftAlternate && NP >= 16)
+        return spread_soft(p, 2 * (SOFT - kSoftAlternate) + 1);
     constexpr int G = soft_group(NP);
     constexpr int base = SOFT >= kSoftAlternate ? SOFT - kSoftAlternate + PHASE / G : SOFT;
     return (NP >= 8 ? (p & 7) : (PHASE % G) * NP + p) < base;
@@ -321,15 +335,15 @@ __device__ __forceinline__ void pair_update(float2 r2, float2 q2, float2 qs2, fl
 //   SQUARE_I (3D):  r2 = pi^2 + pk   (pi = dz of the two points, pk = dx^2 + dy^2)
 //   else (2D):      r2 = pk^2 + pi   (pk = dx, pi = dy^2 + dz^2 of the two rows)
 // Only the first ZA <= ZH lane pairs are evaluated (the rest of a tile that overhangs the grid);
-// HALF marks pair ZA - 1 as holding one point.
-template <bool SQUARE_I, int XP, int ZH, int ZA, int SOFT, int PHASE, bool HALF, int K = 0, int I = 0>
+// HALF marks pair ZA - 1 as holding one point.  The pairs are the tile's from P0 on.
+template <bool SQUARE_I, int XP, int ZH, int ZA, int SOFT, int PHASE, bool HALF, int P0 = 0, int K = 0, int I = 0>
 __device__ __forceinline__ void pair_rows(const float (&pk)[XP], const float2 (&pi)[ZH], float2 q2, float2 qs2,
                                           float2 (&acc)[XP][ZH])
 {
     static_assert(ZA >= 1 && ZA <= ZH, "active pairs within the tile");
     if constexpr (K < XP) {
         if constexpr (I < ZA) {
-            constexpr bool soft = SOFT != 0 && pair_is_soft<SOFT, XP * ZH, PHASE>(K * ZH + I);
+            constexpr bool soft = SOFT != 0 && pair_is_soft<SOFT, XP * ZH, PHASE>(K * ZH + P0 + I);
             constexpr bool half = HALF && I == ZA - 1;
             if constexpr (half) {
                 const float r2 = SQUARE_I ? fmaf(pi[I].x, pi[I].x, pk[K]) : fmaf(pk[K], pk[K], pi[I].x);
@@ -339,9 +353,9 @@ __device__ __forceinline__ void pair_rows(const float (&pk)[XP], const float2 (&
                                            : __ffma2_rn(splat(pk[K]), splat(pk[K]), pi[I]);
                 pair_update<soft, false>(r2, q2, qs2, acc[K][I]);
             }
-            pair_rows<SQUARE_I, XP, ZH, ZA, SOFT, PHASE, HALF, K, I + 1>(pk, pi, q2, qs2, acc);
+            pair_rows<SQUARE_I, XP, ZH, ZA, SOFT, PHASE, HALF, P0, K, I + 1>(pk, pi, q2, qs2, acc);
         } else {
-            pair_rows<SQUARE_I, XP, ZH, ZA, SOFT, PHASE, HALF, K + 1, 0>(pk, pi, q2, qs2, acc);
+            pair_rows<SQUARE_I, XP, ZH, ZA, SOFT, PHASE, HALF, P0, K + 1, 0>(pk, pi, q2, qs2, acc);
         }
     }
 }

@@ -32,6 +32,35 @@ __device__ __forceinline__ double* shared_sums(unsigned char* tiles)
 }
 inline size_t shared_sums_bytes(int threads, int points) { return static_cast<size_t>(threads) * points * sizeof(double); }
 
+// Record tiles: with 2 x 16 points a thread, each warp of a 3D tile turns 24 atoms at a time into records
+// in its own part of shared memory -- x, y, q, q * kSoftRsqrtScale and the atom's z differences to the
+// tile's 16 planes -- and evaluates them from there (record_accumulate), so the pair loop spends nothing
+// on dz and a thread's 32 points share what is left of an atom's cost.  Only tiles of this shape: with 16
+// points a thread the records' loads cost what they save (5.76 Tpair/s in a bare pair loop against
+// 5.87), with 64 the registers leave 12 warps an SM (5.88 against 6.30 with 32).
+constexpr int kRecordAtoms = 24;
+constexpr int kRecordMerge = 48;  // atoms per FP32 partial of the FP64-merge forms
+constexpr bool record_tile(const int zi, const int xp, const int src, const int soa, const int prec, const int mode)
+{
+    return mode == kModeGrid3d && src == kSrcShared && soa == 0 && zi == 16 && xp == 2 &&
+           (prec == kPrecFp32 || prec == kPrecFp64Merge || prec == kPrecFp64MergeShared);
+}
+constexpr int record_floats(const int zi) { return 4 + zi; }                                      // one atom
+constexpr int record_warp_floats(const int zi) { return kRecordAtoms * record_floats(zi) + zi; }  // and the planes' z
+constexpr int kRecordSplitWarps = 8;  // record tiles of small maps: warps of a CTA that share a tile's atoms
+
+// Dynamic shared memory of the forms with one CTA per tile and of the batched kernel: the TMA ring and
+// its barriers, or the records of a record tile, and after them the FP64 sums of kPrecFp64MergeShared.
+inline size_t tile_smem_bytes(const int threads, const int zi, const int xp, const int soa, const int prec, const int mode)
+{
+    size_t bytes = kStages * kTileAtoms * 16 + kStages * 8;
+    if (record_tile(zi, xp, kSrcShared, soa, prec, mode))
+        bytes = static_cast<size_t>((threads + 31) / 32) * record_warp_floats(zi) * sizeof(float);
+    if (prec == kPrecFp64MergeShared)
+        bytes += shared_sums_bytes(threads, zi * xp);
+    return bytes;
+}
+
 // Cluster sizes of the atom-split form: 2..8 are portable; 9..16 use the B200's non-portable
 // cluster sizes (opted into per kernel; refused with a device-limits error where the block does not fit).
 constexpr int kMaxPortableSplit = 8;
@@ -58,6 +87,9 @@ struct FwdLaunch {
     size_t smem;
     int vec_store;  // 1 if x-vector stores are aligned for this launch
     int split;      // atom split: chunks of the atoms per point tile (0 / 1 = none)
+    int record_group;  // record tiles with their atoms split: warps of a CTA per tile (0: not split)
+    int record_ranks;  // CTAs per tile
+    int record_depth;  // planes per tile, ZI or ZI / 2
     SplitQueue queue;  // the queue form's device memory (unused by the other forms)
 };
 
@@ -135,6 +167,156 @@ __device__ __forceinline__ void store_points(float* __restrict__ row, int x0, in
                     row[x0 + k] = accumulate ? row[x0 + k] + v[k] : v[k];
         }
     }
+}
+
+// The first `count` records of a batch against a thread's columns: its first D planes, which are the
+// tile's from 2 * M0 on (the soft / MUFU choice goes by a plane's place among the tile's ZI).
+template <int XP, int ZI, int M0, int D, int SOFT>
+__device__ __forceinline__ void record_batch(const float4* rec, const int count, const float (&gx)[XP], const float gy,
+                                             float2 (&acc)[XP][ZI / 2])
+{
+#pragma unroll 1
+    for (int j = 0; j < count; ++j) {
+        const float4* r = rec + j * (record_floats(ZI) / 4);
+        const float4 a = r[0];  // x, y, q, scaled q
+        const float dy = gy - a.y;
+        const float dy2 = dy * dy;
+        float2 dz[ZI / 2];
+#pragma unroll
+        for (int m = 0; m < (D + 3) / 4; ++m) {
+            const float4 d = r[1 + m];
+            dz[2 * m] = make_float2(d.x, d.y);
+            dz[2 * m + 1] = make_float2(d.z, d.w);
+        }
+        float dxy[XP];
+#pragma unroll
+        for (int k = 0; k < XP; ++k) {
+            const float dx = gx[k] - a.x;
+            dxy[k] = fmaf(dx, dx, dy2);
+        }
+        pair_rows<true, XP, ZI / 2, D / 2, SOFT, 0, false, M0>(dxy, dz, splat(a.z), splat(a.w), acc);
+    }
+}
+
+// The atoms [a0, a1) (a0 a multiple of kRecordMerge) through a warp's records in `rec`, the tile's planes
+// from z0 on, `pairs` pairs of them (of a whole tile, or with HALVES of its sub-th half); merge() after
+// every kRecordMerge atoms and at the end.  The lanes load the next batch of atoms into registers while
+// the warp evaluates the current one.
+template <int ZI, int XP, int SOFT, bool HALVES, class Merge>
+__device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, const int lane, const int lanes, const int z0,
+                                             const int pairs, const int sub, const int64_t a0, const int64_t a1,
+                                             const float (&gx)[XP], const float gy, float2 (&acc)[XP][ZI / 2], Merge&& merge)
+{
+    constexpr int ZH = ZI / 2;
+    static_assert(soft_phases(SOFT, XP * ZH) == 1 && kRecordMerge == 2 * kRecordAtoms, "one pattern, two batches a partial");
+    float4* planes_z = rec + kRecordAtoms * record_floats(ZI) / 4;
+    __syncwarp();  // a persistent kernel's previous tile has been read
+    for (int m = lane; m < ZI; m += lanes)
+        reinterpret_cast<float*>(planes_z)[m] = fmaf(static_cast<float>(z0 + m), p.h, p.oz);
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 next = lane < kRecordAtoms && a0 + lane < a1 ? p.atoms[a0 + lane] : none;
+    bool odd = false;
+    for (int64_t b = a0; b < a1; b += kRecordAtoms) {
+        const int count = static_cast<int>(a1 - b < kRecordAtoms ? a1 - b : kRecordAtoms);
+        __syncwarp();  // the previous records have been read
+        for (int j = lane; j < count; j += lanes) {
+            const float4 a = j == lane ? next : p.atoms[b + j];
+            float4* r = rec + j * (record_floats(ZI) / 4);
+            r[0] = make_float4(a.x, a.y, a.w, a.w * kSoftRsqrtScale);
+#pragma unroll
+            for (int m = 0; m < ZI / 4; ++m) {
+                const float4 z = planes_z[m];
+                r[1 + m] = make_float4(z.x - a.z, z.y - a.z, z.z - a.z, z.w - a.z);
+            }
+        }
+        __syncwarp();
+        if (lane < kRecordAtoms && b + kRecordAtoms + lane < a1)
+            next = p.atoms[b + kRecordAtoms + lane];
+        if (HALVES && sub != 0)
+            with_phase<ZH / 2>(pairs - 1, [&](auto q) {
+                record_batch<XP, ZI, ZH / 2, 2 * (decltype(q)::value + 1), SOFT>(rec, count, gx, gy, acc);
+            });
+        else if (pairs == ZH)
+            record_batch<XP, ZI, 0, ZI, SOFT>(rec, count, gx, gy, acc);
+        else
+            with_phase<ZH - 1>(pairs - 1, [&](auto q) {
+                record_batch<XP, ZI, 0, 2 * (decltype(q)::value + 1), SOFT>(rec, count, gx, gy, acc);
+            });
+        if (odd)
+            merge();
+        odd = !odd;
+    }
+    if (odd)
+        merge();
+}
+
+// tile_accumulate for record tiles: a warp needs no other.  On 256^3 x 65,536 with 5/16 of the roots on
+// the FMA pipe: FP32 sums 180.1 ms = 6.10 Tpair/s (8 x 2 points through the TMA ring, 2/8: 191.8 ms), FP64
+// merge 187.4 ms = 5.87 Tpair/s (195.9).  An FP32 partial of 48 atoms, not kMergeAtoms: the shorter sums
+// take back what the larger share of FMA-pipe roots adds to the error (64-bit error of a 128^3 map
+// 2.49e-7; 8 x 2 points with 64 atoms and 2/8: 2.58e-7; 96 atoms 2 % faster but 3.00e-7, 32 atoms 2 %
+// slower, 6/16 with 48 1 % faster but 2.61e-7).
+template <int ZI, int XP, int PREC, int SOFT>
+__device__ __forceinline__ void record_accumulate(const FwdParams& p, const int x0, const int yrow, const int z0,
+                                                  unsigned char* smem, float (&val)[XP][ZI])
+{
+    constexpr int ZH = ZI / 2;
+    const int threads = blockDim.x * blockDim.y;
+    const int t = threadIdx.y * blockDim.x + threadIdx.x;
+    const int warps = (threads + 31) / 32;
+    const int lanes = threads - t / 32 * 32 < 32 ? threads - t / 32 * 32 : 32;  // a block's last warp may be partial
+    float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem) + t / 32 * record_warp_floats(ZI));
+    // FP64 sums: thread-private, in shared memory after the warps' records or in registers
+    double* sums = reinterpret_cast<double*>(reinterpret_cast<float*>(smem) + warps * record_warp_floats(ZI)) + t;
+    double sum64[PREC == kPrecFp64Merge ? XP * ZI : 1];
+#pragma unroll
+    for (int i = 0; i < XP * ZI; ++i) {
+        if constexpr (PREC == kPrecFp64MergeShared)
+            sums[i * threads] = 0.0;
+        else if constexpr (PREC == kPrecFp64Merge)
+            sum64[i] = 0.0;
+    }
+    float gx[XP];
+#pragma unroll
+    for (int k = 0; k < XP; ++k)
+        gx[k] = fmaf(static_cast<float>(x0 + k), p.h, p.ox);
+    const float gy = fmaf(static_cast<float>(yrow), p.h, p.oy);
+    float2 acc[XP][ZH];
+    auto clear = [&]() {
+#pragma unroll
+        for (int k = 0; k < XP; ++k)
+#pragma unroll
+            for (int i = 0; i < ZH; ++i)
+                acc[k][i] = make_float2(0.0f, 0.0f);
+    };
+    clear();
+    // a tile that overhangs the grid evaluates its planes inside it, in pairs of planes
+    const int pairs = p.nz - z0 < ZI ? (p.nz - z0 + 1) / 2 : ZH;
+    record_range<ZI, XP, SOFT, false>(p, rec, t % 32, lanes, z0, pairs, 0, 0, p.n_atoms, gx, gy, acc, [&]() {
+        if constexpr (PREC != kPrecFp32) {
+#pragma unroll
+            for (int k = 0; k < XP; ++k)
+#pragma unroll
+                for (int m = 0; m < ZI; ++m) {
+                    if constexpr (PREC == kPrecFp64MergeShared)
+                        sums[(k * ZI + m) * threads] += static_cast<double>(coul::lane(acc[k][m / 2], m & 1));
+                    else
+                        sum64[k * ZI + m] += static_cast<double>(coul::lane(acc[k][m / 2], m & 1));
+                }
+            clear();
+        }
+    });
+#pragma unroll
+    for (int k = 0; k < XP; ++k)
+#pragma unroll
+        for (int m = 0; m < ZI; ++m) {
+            if constexpr (PREC == kPrecFp64MergeShared)
+                val[k][m] = static_cast<float>(sums[(k * ZI + m) * threads]);
+            else if constexpr (PREC == kPrecFp64Merge)
+                val[k][m] = static_cast<float>(sum64[k * ZI + m]);
+            else
+                val[k][m] = coul::lane(acc[k][m / 2], m & 1);
+        }
 }
 
 // Shared-memory ring of the TMA-staged atom stream: kStages stages of kTileAtoms float4 (or four
@@ -474,18 +656,22 @@ __device__ __forceinline__ bool tile_pass(const FwdParams& p, const int x0, cons
                                           unsigned char* tiles, uint64_t* full, uint32_t& gstage)
 {
     float val[XP][ZI];
-    if (!tile_accumulate<ZI, XP, UNR, SRC, SOA, PREC, SOFT, MODE, ZTRIM>(p, x0, yrow, z0, tiles, full, gstage, val))
-        return false;
+    if constexpr (record_tile(ZI, XP, SRC, SOA, PREC, MODE)) {
+        record_accumulate<ZI, XP, PREC, SOFT>(p, x0, yrow, z0, tiles, val);
+    } else {
+        if (!tile_accumulate<ZI, XP, UNR, SRC, SOA, PREC, SOFT, MODE, ZTRIM>(p, x0, yrow, z0, tiles, full, gstage, val))
+            return false;
+    }
     store_tile<ZI, XP, MODE>(p, x0, yrow, z0, vec_ok, val);
     return true;
 }
 
 // Resident 256-thread blocks the register budget of fwd_kernel is sized for: with its FP64 sums in
-// shared memory a thread of up to 16 points fits in 51 registers (five such blocks per SM); otherwise
-// the compiler's choice.
+// shared memory a thread of up to 16 points fits in 51 registers (five such blocks per SM), one of 32
+// in 128 (two); otherwise the compiler's choice.
 constexpr int fwd_min_blocks(const int prec, const int points)
 {
-    return prec == kPrecFp64MergeShared && points <= 16 ? 5 : 1;
+    return prec == kPrecFp64MergeShared ? (points <= 16 ? 5 : points <= 32 ? 2 : 1) : 1;
 }
 
 // The x-y tiles of a 3D map are linear where the block's own rectangles would be padded more: the
@@ -525,7 +711,10 @@ __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) fw
         }
     }
     uint32_t gstage = 0;
-    if constexpr (SRC == kSrcShared) {
+    if constexpr (record_tile(ZI, XP, SRC, SOA, PREC, MODE)) {
+        extern __shared__ __align__(128) unsigned char smem_raw[];
+        (void)tile_pass<ZI, XP, UNR, SRC, SOA, PREC, SOFT, MODE>(p, x0, yrow, z0, vec_ok, smem_raw, nullptr, gstage);
+    } else if constexpr (SRC == kSrcShared) {
         extern __shared__ __align__(128) unsigned char smem_raw[];
         uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + kStages * kTileAtoms * 16);
         ring_init(full, threadIdx.y * blockDim.x + threadIdx.x);
@@ -533,6 +722,115 @@ __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) fw
     } else {
         (void)tile_pass<ZI, XP, UNR, SRC, SOA, PREC, SOFT, MODE>(p, x0, yrow, z0, vec_ok, nullptr, nullptr, gstage);
     }
+}
+
+// FP64-merge record tiles with their atoms split: GROUP (8, 4 or 2) of a CTA's eight warps, and with all
+// eight the CTAs of a cluster, share a tile of 32 linear columns by `depth` planes (ZI or half of it).
+// They split its atoms at multiples of kRecordMerge, so they form the FP32 partials of the whole tile and
+// only the FP64 additions of those take another order (warp order, then rank order): a point's float is
+// that of fwd_kernel unless its FP64 sum lies within a few units of the 53rd bit of a rounding boundary.
+// How a map is split follows from the whole grid and the atom count, so slabs equal the map bit for bit.
+// One warp a tile leaves a 128^3 map 3.5 warps a scheduler and its last ones alone (3,573 us x 8,192
+// atoms; split over eight 2,948), a 64^3 map half of the SMs idle (670 and 224 us x 4,000 atoms); even
+// 256^3 x 65,536 gains from the shorter tail (187.5 and 184.1 ms).
+template <int ZI, int XP, int SOFT, int GROUP>
+__global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel(const FwdParams p, const int depth,
+                                                                                const int vec_ok)
+{
+    constexpr int ZH = ZI / 2;
+    constexpr int P = XP * ZI;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int lane = threadIdx.x % 32;
+    const int warp = threadIdx.x / 32;
+    const int ranks = static_cast<int>(cluster_size());
+    const int rank = static_cast<int>(cluster_rank());
+    const int gw = warp % GROUP;      // this warp among those of its tile
+    const int first = warp - gw;      // and the first of them
+    float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem_raw) + warp * record_warp_floats(ZI));
+    double* all = reinterpret_cast<double*>(reinterpret_cast<float*>(smem_raw) + kRecordSplitWarps * record_warp_floats(ZI));
+    double* sums = all + warp * P * 32 + lane;
+    const int64_t tile = static_cast<int64_t>(blockIdx.x / ranks) * (kRecordSplitWarps / GROUP) + warp / GROUP;
+    const int64_t column = tile * 32 + lane;
+    const int yrow = static_cast<int>(column / p.columns);
+    const int x0 = static_cast<int>(column % p.columns) * XP;
+    const int plane0 = static_cast<int>(blockIdx.y) * depth;
+    const int z0 = p.z_base + plane0;
+    const int planes = p.nz - z0 < depth ? p.nz - z0 : depth;
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+        sums[i * 32] = 0.0;
+    float gx[XP];
+#pragma unroll
+    for (int k = 0; k < XP; ++k)
+        gx[k] = fmaf(static_cast<float>(x0 + k), p.h, p.ox);
+    const float gy = fmaf(static_cast<float>(yrow), p.h, p.oy);
+    float2 acc[XP][ZH];
+    auto clear = [&]() {
+#pragma unroll
+        for (int k = 0; k < XP; ++k)
+#pragma unroll
+            for (int i = 0; i < ZH; ++i)
+                acc[k][i] = make_float2(0.0f, 0.0f);
+    };
+    clear();
+    // this warp's share: whole partials
+    const int64_t partials = (p.n_atoms + kRecordMerge - 1) / kRecordMerge;
+    const int64_t shares = static_cast<int64_t>(ranks) * GROUP;
+    const int64_t w = static_cast<int64_t>(rank) * GROUP + gw;
+    const int64_t a0 = (partials / shares * w + partials % shares * w / shares) * kRecordMerge;
+    const int64_t stop = (partials / shares * (w + 1) + partials % shares * (w + 1) / shares) * kRecordMerge;
+    record_range<ZI, XP, SOFT, true>(p, rec, lane, 32, z0, (planes + 1) / 2, plane0 % ZI / depth, a0,
+                                     stop < p.n_atoms ? stop : p.n_atoms, gx, gy, acc, [&]() {
+#pragma unroll
+        for (int m = 0; m < ZI; ++m) {
+            if (m < planes) {
+#pragma unroll
+                for (int k = 0; k < XP; ++k)
+                    sums[(m * XP + k) * 32] += static_cast<double>(coul::lane(acc[k][m / 2], m & 1));
+            }
+        }
+        clear();
+    });
+    __syncthreads();
+    // a row of XP points per warp at a time: the warps' sums in warp order, the ranks' in rank order
+    double* mine = all + first * P * 32 + lane;
+    for (int m = gw; m < planes; m += GROUP) {
+#pragma unroll
+        for (int k = 0; k < XP; ++k) {
+            double sum = mine[(m * XP + k) * 32];
+#pragma unroll
+            for (int v = 1; v < GROUP; ++v)
+                sum += mine[(v * P + m * XP + k) * 32];
+            mine[(m * XP + k) * 32] = sum;  // only this thread reads or writes this entry
+        }
+    }
+    if (ranks > 1)
+        cluster_sync();
+    for (int m = gw * ranks + rank; m < planes; m += GROUP * ranks) {
+        float v[XP];
+#pragma unroll
+        for (int k = 0; k < XP; ++k) {
+            const double* e = mine + (m * XP + k) * 32;
+            double sum = *e;
+            if (ranks > 1) {
+                sum = ld_cluster_f64(cluster_map(e, 0));
+                for (int r = 1; r < ranks; ++r)
+                    sum += ld_cluster_f64(cluster_map(e, static_cast<uint32_t>(r)));
+            }
+            v[k] = static_cast<float>(sum);
+        }
+        if (yrow < p.ny)
+            store_points<XP>(p.out + (static_cast<int64_t>(z0 + m - p.z_base) * p.ny + yrow) * p.nx, x0, p.nx, v,
+                             p.accumulate, vec_ok);
+    }
+    if (ranks > 1)
+        cluster_sync();  // the sums stay valid until every rank has read its share
+}
+
+inline size_t record_split_smem_bytes(const int zi, const int xp)
+{
+    return static_cast<size_t>(kRecordSplitWarps) * record_warp_floats(zi) * sizeof(float) +
+           shared_sums_bytes(32 * kRecordSplitWarps, zi * xp);
 }
 
 // Stores value i = (k * ZI + m) * nthreads + t of a tile's register blocks -- thread t's k-th x point,
@@ -1087,6 +1385,30 @@ cudaError_t launch_fwd(const FwdLaunch& L, cudaStream_t stream)
         } while (off < n);
         return cudaSuccess;
     } else {
+        if constexpr (record_tile(ZI, XP, SRC, SOA, PREC, MODE) && PREC != kPrecFp32) {
+            if (L.record_group > 0) {
+                auto split = L.record_group == 8   ? record_split_kernel<ZI, XP, SOFT, 8>
+                             : L.record_group == 4 ? record_split_kernel<ZI, XP, SOFT, 4>
+                                                   : record_split_kernel<ZI, XP, SOFT, 2>;
+                const cudaError_t e = cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           static_cast<int>(L.smem));
+                if (e != cudaSuccess)
+                    return e;
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = L.grid;
+                cfg.blockDim = dim3(32 * kRecordSplitWarps, 1, 1);
+                cfg.dynamicSmemBytes = L.smem;
+                cfg.stream = stream;
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = static_cast<unsigned>(L.record_ranks);
+                attr[0].val.clusterDim.y = 1;
+                attr[0].val.clusterDim.z = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = L.record_ranks > 1 ? 1 : 0;
+                return cudaLaunchKernelEx(&cfg, split, L.p, L.record_depth, L.vec_store);
+            }
+        }
         if (L.smem > 48u * 1024u) {
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        static_cast<int>(L.smem));

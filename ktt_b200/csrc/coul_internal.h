@@ -51,7 +51,9 @@ int ctx_end_timing(coul_ctx* ctx);
 bool aligned16(const void* p);
 int validate_tune(const coul_tune* t, int mode, int soa, const VariantEntry** out);
 int validate_grid(const coul_grid* g);
-int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t);
+// nz: planes of the whole grid, by which a small 3D map's atoms are split over more CTAs (prm.z_base and
+// prm.nz bound the slab); 0: one warp runs through all atoms of a tile, as in the batched kernel.
+int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz);
 int queue_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const coul_tune* t);
 int balanced_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const coul_tune* t);
 // Releases the device resources of the context's live batches and detaches them (coul_batched.cu);

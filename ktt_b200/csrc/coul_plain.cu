@@ -55,8 +55,6 @@ struct PlainParams {
     int vec_ok;
 };
 
-__host__ __device__ constexpr bool spread_soft(int p, int soft) { return (p + 1) * soft / 16 != p * soft / 16; }
-
 // This warp's share of the atoms: the w-th of all warps of all CTAs that share the tile.
 __device__ __forceinline__ void warp_atoms(const int64_t n, const uint32_t ranks, int64_t& begin, int64_t& end)
 {

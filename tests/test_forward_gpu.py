@@ -344,3 +344,38 @@ def test_linear_and_rectangular_tiles(ctx, dims, tune):
     assert errors.report(_np(out), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
     row = ktt_b200.Tune(**dict(tune.as_dict(), block_x=1, block_y=1))
     assert torch.equal(out, ctx.forward_3d(_t(a), dims, h, origin, tune=row))
+
+
+@pytest.mark.parametrize("n", [0, 1, 23, 24, 25, 48, 191, 193, 400])
+@pytest.mark.parametrize("block", [(32, 4), (7, 3), (16, 1), (64, 4)])
+@pytest.mark.parametrize("nz", [7, 8, 9, 33])
+def test_record_tiles(ctx, n, block, nz):
+    """2 x 16 points a thread, atoms as records in shared memory: atom counts around the batches (24), the
+    FP32 partials (48) and the stages (192), blocks with a partial warp, depths that use half a tile;
+    within the norm tolerance of the oracle, FP64 sums in registers and in shared memory bit for bit
+    alike, slabs equal to the map."""
+    import torch
+    a = np.empty((n, 4), dtype=np.float32)
+    rng = np.random.default_rng(n + nz)
+    a[:, :3] = rng.uniform(0.0, 18.0, (n, 3))
+    a[:, 3] = rng.uniform(-1.0, 1.0, n)
+    atoms = _t(a) if n else torch.zeros((0, 4), device="cuda")
+    dims, h, origin = (35, 11, nz), 0.5, (-1.0, 0.5, 2.0)
+    ref = oracle.grid3d(a, h, dims, origin) if n else None
+    maps = {}
+    for prec in (ktt_b200.PREC_FP32, ktt_b200.PREC_FP64_MERGE, ktt_b200.PREC_FP64_MERGE_SHARED):
+        for soft in (2, 12):
+            tune = ktt_b200.Tune(block_x=block[0], block_y=block[1], z_iterations=16, x_points=2, precision=prec,
+                                 rsqrt_soft=soft)
+            out = torch.full((nz, 11, 35), float("nan"), device="cuda")
+            ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=out)
+            if n:
+                assert errors.report(_np(out), ref)["rel_norm"] <= TOL_NORM
+            else:
+                assert torch.count_nonzero(out) == 0
+            if nz > 16:
+                slab = ctx.forward_3d_slab(atoms, dims, h, 16, nz, origin, tune=tune)
+                assert torch.equal(slab, out[16:])
+            maps[prec, soft] = out
+    for soft in (2, 12):
+        assert torch.equal(maps[ktt_b200.PREC_FP64_MERGE, soft], maps[ktt_b200.PREC_FP64_MERGE_SHARED, soft])
