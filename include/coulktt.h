@@ -337,6 +337,10 @@ COUL_API int coul_nbody_tune_supported(const coul_nbody_tune* tune);
 COUL_API int coul_nbody_step(coul_ctx* ctx, const float* d_pos_mass, const float* d_vel, int64_t n, float dt,
                              float damping, float softening_sqr, const coul_nbody_tune* tune, float* d_pos_mass_new,
                              float* d_vel_new);
+/* The same step without a configuration: a kernel that suits every body count (csrc/coul_nbody.cu).  No
+   counterpart in the reference, whose tuner picks a configuration for every launch. */
+COUL_API int coul_nbody_step_plain(coul_ctx* ctx, const float* d_pos_mass, const float* d_vel, int64_t n, float dt,
+                                   float damping, float softening_sqr, float* d_pos_mass_new, float* d_vel_new);
 
 /* ---- batched: many molecules in one persistent launch ------------------------------ */
 /*

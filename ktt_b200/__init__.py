@@ -432,7 +432,8 @@ def nbody_tune_supported(tune: NbodyTune) -> bool:
 def nbody_step(ctx: "CoulombContext", pos_mass, vel, dt: float, damping: float, softening_sqr: float,
                tune: NbodyTune | None = None, out_pos=None, out_vel=None):
     """One step of KTT's N-body example (coul_nbody_step): pos_mass and vel are (n, 4) float32 CUDA
-    tensors; returns (pos_mass', vel')."""
+    tensors; returns (pos_mass', vel').  Without a tune the library's plain step kernel runs
+    (coul_nbody_step_plain)."""
     import torch
     CoulombContext._check_atoms(pos_mass)
     CoulombContext._check_atoms(vel)
@@ -442,7 +443,11 @@ def nbody_step(ctx: "CoulombContext", pos_mass, vel, dt: float, damping: float, 
     out_pos = torch.empty_like(pos_mass) if out_pos is None else out_pos
     out_vel = torch.empty_like(vel) if out_vel is None else out_vel
     ctx._bind_stream()
-    t = (tune or NbodyTune()).c()
+    if tune is None:
+        _check(ctx._lib.coul_nbody_step_plain(ctx.handle, _ptr(pos_mass), _ptr(vel), n, float(dt), float(damping),
+                                              float(softening_sqr), _ptr(out_pos), _ptr(out_vel)))
+        return out_pos, out_vel
+    t = tune.c()
     _check(ctx._lib.coul_nbody_step(ctx.handle, _ptr(pos_mass), _ptr(vel), n, float(dt), float(damping),
                                     float(softening_sqr), ctypes.byref(t), _ptr(out_pos), _ptr(out_vel)))
     return out_pos, out_vel

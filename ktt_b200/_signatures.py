@@ -29,6 +29,7 @@ def register(lib) -> None:
         "coul_nbody_tune_supported": [ctypes.POINTER(NbodyTuneC)],
         "coul_nbody_step": [vp, vp, vp, ctypes.c_int64, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                             ctypes.POINTER(NbodyTuneC), vp, vp],
+        "coul_nbody_step_plain": [vp, vp, vp, ctypes.c_int64, ctypes.c_float, ctypes.c_float, ctypes.c_float, vp, vp],
         "coul_buffer_alloc": [vp, ctypes.c_size_t, ctypes.POINTER(vp)],
         "coul_buffer_free": [vp, vp],
         "coul_buffer_upload": [vp, vp, vp, ctypes.c_size_t],

@@ -31,6 +31,7 @@ struct coul_ctx {
     std::vector<std::function<void()>> cleanups;  // frees buffers owned by other units (run at destroy)
     void* adjoint_workspace = nullptr;            // FP64 partials of coul_adjoint_3d (coul_adjoint.cu)
     void* split_workspace_state = nullptr;        // partial blocks and counters of the queue and balanced forms
+    void* nbody_workspace = nullptr;              // partial accelerations of the pair form (coul_nbody.cu)
     std::vector<coul_batch*> batches;             // live batches (their device resources go with the context)
     struct Occupancy {
         const void* kernel;

@@ -84,3 +84,51 @@ def test_nbody_rejects_bad_arguments(ctx):
         ktt_b200.nbody_step(ctx, tp, tv, DT, DAMPING, EPS2, ktt_b200.NbodyTune(bodies_per_thread=3))
     with pytest.raises(ktt_b200.CoulombError):
         ktt_b200.nbody_step(ctx, tp, tv, DT, DAMPING, EPS2, ktt_b200.NbodyTune(block_x=48))
+
+
+@pytest.mark.parametrize("n", [1, 33, 127, 129, 1000, 4095, 4096, 4097, 5120, 6145, 8192, 9000])
+def test_nbody_plain_step(ctx, n):
+    """Steps without a tune: tiles, shares and clusters of the one-way kernel; odd and even numbers of
+    blocks, a ragged last block and more parts than tiles in the pair form (4,096 bodies on)."""
+    import torch
+    pos, vel = _bodies(n, seed=n)
+    tp, tv = torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda()
+    p, v = ktt_b200.nbody_step(ctx, tp, tv, DT, DAMPING, EPS2)
+    _check(pos, vel, p.cpu().numpy(), v.cpu().numpy())
+    _, a = ktt_b200.nbody_step(ctx, tp, torch.zeros_like(tv), 1.0, DAMPING, EPS2)
+    _, _, ref_acc = oracle.nbody_step(pos, np.zeros_like(vel), 1.0, DAMPING, EPS2)
+    assert np.abs(a.cpu().numpy()[:, :3].astype(np.float64) - ref_acc).max() <= 1e-5 * max(np.abs(ref_acc).max(), 1e-30)
+    p2, v2 = ktt_b200.nbody_step(ctx, tp, tv, DT, DAMPING, EPS2)
+    assert torch.equal(p, p2) and torch.equal(v, v2)
+
+
+def test_nbody_plain_step_on_two_streams_and_captured(ctx):
+    """The pair form's workspace is shared by the context's streams in order (steps of two sizes on two
+    streams, nothing waited for between), and a captured step uses none of it: its replay gives the same
+    accelerations to FP32 rounding after later steps have grown the workspace."""
+    import torch
+    sizes = (9000, 6000)
+    data, want = [], []
+    for n in sizes:
+        pos, vel = _bodies(n, seed=n)
+        data.append((torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda()))
+        want.append(ktt_b200.nbody_step(ctx, *data[-1], DT, DAMPING, EPS2))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for i in range(8):
+        with torch.cuda.stream(streams[i % 2]):
+            got.append((i % 2, ktt_b200.nbody_step(ctx, *data[i % 2], DT, DAMPING, EPS2)))
+    torch.cuda.synchronize()
+    for k, (p, v) in got:
+        assert torch.equal(p, want[k][0]) and torch.equal(v, want[k][1])
+    out = [torch.empty_like(t) for t in data[1]]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ktt_b200.nbody_step(ctx, *data[1], DT, DAMPING, EPS2, out_pos=out[0], out_vel=out[1])
+    pos, vel = _bodies(20000, seed=3)
+    ktt_b200.nbody_step(ctx, torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda(), DT, DAMPING, EPS2)
+    graph.replay()
+    torch.cuda.synchronize()
+    # two summation orders of an acceleration, times dt: 1e-5 of the largest velocity covers both
+    assert float((out[1] - want[1][1]).abs().max()) <= 1e-5 * float(want[1][1].abs().max())
