@@ -482,6 +482,31 @@ static void record_split_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tun
                   static_cast<unsigned>((L.p.nz - L.p.z_base + depth - 1) / depth), 1);
 }
 
+// FP64 pairs: tiles of 32 linear columns, eight warps each, and as many CTAs of a
+// cluster as leave no SM without one while a warp keeps 8 atoms (from the whole grid's nz planes, so that
+// slabs equal the map).
+static int fp64_pairs_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tune* t, int nz)
+{
+    const int zi = fp64_zi(t->z_iterations, t->x_points);
+    const int xp = fp64_xp(t->z_iterations, t->x_points);
+    L.p.columns = (L.p.nx + xp - 1) / xp;
+    const int64_t tiles_xy = (static_cast<int64_t>(L.p.columns) * L.p.ny + 31) / 32;
+    const int64_t tiles = tiles_xy * ((nz + zi - 1) / zi);
+    int ranks = 1;
+    while (ranks < kMaxPortableSplit && tiles * ranks < ctx->sm_count &&
+           L.p.n_atoms >= 2LL * ranks * kRecordSplitWarps * 8)
+        ranks *= 2;
+    if (tiles_xy * ranks > 2147483647LL)
+        return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
+    L.record_ranks = ranks;
+    const int64_t tiles_z = (L.p.nz - L.p.z_base + zi - 1) / zi;
+    if (tiles_z > 65535)
+        return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
+    L.grid = dim3(static_cast<unsigned>(tiles_xy * ranks), static_cast<unsigned>(tiles_z), 1);
+    L.smem = fp64_pairs_smem_bytes(zi, xp);
+    return COUL_OK;
+}
+
 // Launch one forward variant over a grid; shared by the 3D AoS/SoA and 2D entry points and by
 // the batched path's plain-launch baseline.
 int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz)
@@ -519,6 +544,11 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
     L.smem = t->atom_source == COUL_ATOMS_SHARED_TMA
                  ? tile_smem_bytes(t->block_x * t->block_y, t->z_iterations, t->x_points, v->key.soa, t->precision, mode)
                  : 0;
+    if (t->precision == COUL_PREC_FP64_PAIRS) {
+        const int rc = fp64_pairs_setup(ctx, L, t, nz > 0 ? nz : prm.nz);
+        if (rc != COUL_OK)
+            return rc;
+    }
     if (nz > 0 && v->key.split == 0 && t->precision != COUL_PREC_FP32 &&
         record_tile(t->z_iterations, t->x_points, t->atom_source, v->key.soa, t->precision, mode))
         record_split_setup(ctx, L, t, nz);

@@ -416,34 +416,14 @@ __device__ __forceinline__ double rsqrt_mufu_f64(double x)
     return y;
 }
 
-template <int XP, int ZI>
-__device__ __forceinline__ void pair_block_3d_f64(const double (&gx)[XP], double gy, const double (&gz)[ZI], float4 a,
-                                                  double (&acc)[XP][ZI])
+// acc + q / sqrt(dz^2 + dxy)
+__device__ __forceinline__ double pair_f64(const double dz, const double dxy, const double q, const double acc)
 {
-    const double dy = gy - static_cast<double>(a.y);
-    const double dy2 = dy * dy;
-    const double q = static_cast<double>(a.w);
-    double dxy[XP];
-#pragma unroll
-    for (int k = 0; k < XP; ++k) {
-        const double dx = gx[k] - static_cast<double>(a.x);
-        dxy[k] = fma(dx, dx, dy2);
-    }
-    double dz[ZI];
-#pragma unroll
-    for (int m = 0; m < ZI; ++m)
-        dz[m] = gz[m] - static_cast<double>(a.z);
-#pragma unroll
-    for (int k = 0; k < XP; ++k) {
-#pragma unroll
-        for (int m = 0; m < ZI; ++m) {
-            const double r2 = fma(dz[m], dz[m], dxy[k]);
-            double y = rsqrt_mufu_f64(r2);
-            const double e = fma(-r2, y * y, 1.0);
-            y = fma(y * e, 0.5, y);
-            acc[k][m] = fma(q, y, acc[k][m]);
-        }
-    }
+    const double r2 = fma(dz, dz, dxy);
+    double y = rsqrt_mufu_f64(r2);
+    const double e = fma(-r2, y * y, 1.0);
+    y = fma(y * e, 0.5, y);
+    return fma(q, y, acc);
 }
 
 // Knuth's two-sum: s + e == a + b exactly (round-to-nearest, no contraction of additions).

@@ -346,8 +346,8 @@ __device__ __forceinline__ bool tile_accumulate(const FwdParams& p, const int x0
                                                 unsigned char* tiles, uint64_t* full, uint32_t& gstage,
                                                 float (&val)[XP][ZI], const uint32_t phase_base = 0)
 {
-    static_assert(!ZTRIM || (MODE == kModeGrid3d && SRC == kSrcShared && PREC != kPrecFp64Pairs),
-                  "z trimming: 3D maps, shared-memory atoms, FP32 pairs");
+    static_assert(PREC != kPrecFp64Pairs, "FP64 pairs have their own kernel");
+    static_assert(!ZTRIM || (MODE == kModeGrid3d && SRC == kSrcShared), "z trimming: 3D maps, shared-memory atoms");
     static_assert(XP == 1 || XP == 2 || XP == 4 || XP == 8, "XP must be 1, 2, 4 or 8");
     // atoms per FP32 partial of the compensated / FP64-merge forms, and the ragged stage's granularity
     constexpr int SUB =
@@ -372,21 +372,6 @@ __device__ __forceinline__ bool tile_accumulate(const FwdParams& p, const int x0
     float2 part[XP][ZH];
     float2 cmp[XP][ZH];
     double acc64[XP][2 * ZH];
-    // FP64 pairs: the point coordinates widened once (3D only)
-    static_assert(PREC != kPrecFp64Pairs || (MODE == kModeGrid3d && SOFT == 0 && SRC == kSrcShared),
-                  "FP64 pairs: 3D maps, MUFU estimate, shared-memory atoms");
-    double gxd[XP], gzd[ZI], accd[XP][ZI];
-    const double gyd = static_cast<double>(gy);
-#pragma unroll
-    for (int k = 0; k < XP; ++k)
-        gxd[k] = static_cast<double>(gx[k]);
-#pragma unroll
-    for (int m = 0; m < ZI; ++m) {
-        gzd[m] = static_cast<double>(lane(gb[m / 2], m & 1));
-#pragma unroll
-        for (int k = 0; k < XP; ++k)
-            accd[k][m] = 0.0;
-    }
 #pragma unroll
     for (int k = 0; k < XP; ++k)
 #pragma unroll
@@ -555,11 +540,7 @@ __device__ __forceinline__ bool tile_accumulate(const FwdParams& p, const int x0
             };
             // the stage runs in whole sub-tiles of SUB atoms (ntr atoms: all kTileAtoms, or the ragged
             // last stage rounded up); the whole stage is one phase of the FMA-pipe share's pattern
-            if constexpr (PREC == kPrecFp64Pairs) {
-#pragma unroll UNR
-                for (int j = 0; j < ntr; ++j)
-                    pair_block_3d_f64<XP, ZI>(gxd, gyd, gzd, atom_at(j), accd);
-            } else {
+            {
                 // G: the stage's phase of the FMA-pipe share; LA: the z points the tile evaluates
                 auto stage = [&](auto phase, auto lanes) {
                     constexpr int G = decltype(phase)::value;
@@ -607,8 +588,6 @@ __device__ __forceinline__ bool tile_accumulate(const FwdParams& p, const int x0
         for (int m = 0; m < ZI; ++m) {
             if constexpr (PREC == kPrecFp32)
                 val[k][m] = lane(acc[k][m / 2], m & 1);
-            else if constexpr (PREC == kPrecFp64Pairs)
-                val[k][m] = static_cast<float>(accd[k][m]);
             else if constexpr (PREC == kPrecCompensated)
                 val[k][m] = lane(acc[k][m / 2], m & 1) + lane(cmp[k][m / 2], m & 1);
             else if constexpr (PREC == kPrecFp64MergeShared)
@@ -619,7 +598,6 @@ __device__ __forceinline__ bool tile_accumulate(const FwdParams& p, const int x0
     (void)part;
     (void)cmp;
     (void)acc64;
-    (void)accd;
     (void)sums;
     (void)sum_tid;
     (void)sum_stride;
@@ -724,6 +702,52 @@ __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) fw
     }
 }
 
+// A tile's FP64 sums from the GROUP warps of each CTA that share it (all[warp][(plane * XP + k) * 32 + lane]),
+// a row of XP points per warp at a time: added in warp order, over the cluster's ranks in rank order,
+// rounded and stored.
+template <int XP, int ZI, int GROUP>
+__device__ __forceinline__ void store_split_sums(const FwdParams& p, double* all, const int planes, const int x0,
+                                                 const int yrow, const int z0, const int vec_ok)
+{
+    constexpr int P = XP * ZI;
+    const int lane = threadIdx.x % 32;
+    const int gw = threadIdx.x / 32 % GROUP;
+    const int ranks = static_cast<int>(cluster_size());
+    double* mine = all + (threadIdx.x / 32 - gw) * P * 32 + lane;
+    __syncthreads();
+    for (int m = gw; m < planes; m += GROUP) {
+#pragma unroll
+        for (int k = 0; k < XP; ++k) {
+            double sum = mine[(m * XP + k) * 32];
+#pragma unroll
+            for (int v = 1; v < GROUP; ++v)
+                sum += mine[(v * P + m * XP + k) * 32];
+            mine[(m * XP + k) * 32] = sum;  // only this thread reads or writes this entry
+        }
+    }
+    if (ranks > 1)
+        cluster_sync();
+    for (int m = gw * ranks + static_cast<int>(cluster_rank()); m < planes; m += GROUP * ranks) {
+        float v[XP];
+#pragma unroll
+        for (int k = 0; k < XP; ++k) {
+            const double* e = mine + (m * XP + k) * 32;
+            double sum = *e;
+            if (ranks > 1) {
+                sum = ld_cluster_f64(cluster_map(e, 0));
+                for (int r = 1; r < ranks; ++r)
+                    sum += ld_cluster_f64(cluster_map(e, static_cast<uint32_t>(r)));
+            }
+            v[k] = static_cast<float>(sum);
+        }
+        if (yrow < p.ny)
+            store_points<XP>(p.out + (static_cast<int64_t>(z0 + m - p.z_base) * p.ny + yrow) * p.nx, x0, p.nx, v,
+                             p.accumulate, vec_ok);
+    }
+    if (ranks > 1)
+        cluster_sync();  // the sums stay valid until every rank has read its share
+}
+
 // FP64-merge record tiles with their atoms split: GROUP (8, 4 or 2) of a CTA's eight warps, and with all
 // eight the CTAs of a cluster, share a tile of 32 linear columns by `depth` planes (ZI or half of it).
 // They split its atoms at multiples of kRecordMerge, so they form the FP32 partials of the whole tile and
@@ -744,8 +768,7 @@ __global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel
     const int warp = threadIdx.x / 32;
     const int ranks = static_cast<int>(cluster_size());
     const int rank = static_cast<int>(cluster_rank());
-    const int gw = warp % GROUP;      // this warp among those of its tile
-    const int first = warp - gw;      // and the first of them
+    const int gw = warp % GROUP;  // this warp among those of its tile
     float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem_raw) + warp * record_warp_floats(ZI));
     double* all = reinterpret_cast<double*>(reinterpret_cast<float*>(smem_raw) + kRecordSplitWarps * record_warp_floats(ZI));
     double* sums = all + warp * P * 32 + lane;
@@ -791,46 +814,96 @@ __global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel
         }
         clear();
     });
-    __syncthreads();
-    // a row of XP points per warp at a time: the warps' sums in warp order, the ranks' in rank order
-    double* mine = all + first * P * 32 + lane;
-    for (int m = gw; m < planes; m += GROUP) {
-#pragma unroll
-        for (int k = 0; k < XP; ++k) {
-            double sum = mine[(m * XP + k) * 32];
-#pragma unroll
-            for (int v = 1; v < GROUP; ++v)
-                sum += mine[(v * P + m * XP + k) * 32];
-            mine[(m * XP + k) * 32] = sum;  // only this thread reads or writes this entry
-        }
-    }
-    if (ranks > 1)
-        cluster_sync();
-    for (int m = gw * ranks + rank; m < planes; m += GROUP * ranks) {
-        float v[XP];
-#pragma unroll
-        for (int k = 0; k < XP; ++k) {
-            const double* e = mine + (m * XP + k) * 32;
-            double sum = *e;
-            if (ranks > 1) {
-                sum = ld_cluster_f64(cluster_map(e, 0));
-                for (int r = 1; r < ranks; ++r)
-                    sum += ld_cluster_f64(cluster_map(e, static_cast<uint32_t>(r)));
-            }
-            v[k] = static_cast<float>(sum);
-        }
-        if (yrow < p.ny)
-            store_points<XP>(p.out + (static_cast<int64_t>(z0 + m - p.z_base) * p.ny + yrow) * p.nx, x0, p.nx, v,
-                             p.accumulate, vec_ok);
-    }
-    if (ranks > 1)
-        cluster_sync();  // the sums stay valid until every rank has read its share
+    store_split_sums<XP, ZI, GROUP>(p, all, planes, x0, yrow, z0, vec_ok);
 }
 
 inline size_t record_split_smem_bytes(const int zi, const int xp)
 {
     return static_cast<size_t>(kRecordSplitWarps) * record_warp_floats(zi) * sizeof(float) +
            shared_sums_bytes(32 * kRecordSplitWarps, zi * xp);
+}
+
+// FP64 pairs (pair math: pair_f64): a warp evaluates a tile of 32 linear columns by ZI planes against its
+// share of the atoms, the eight warps of a CTA (and the CTAs of a cluster, where tiles are few) sharing
+// the tile.  The lanes widen 32 atoms at a time and write them to the warp's shared memory with their z
+// differences to the tile's planes, so the conversions and the dz run once an atom and warp instead of
+// once an atom and thread.  Bound: the FP64 pipe, six operations a pair (2.83e12 pairs/s).  192^3 x 8,192
+// atoms: 2.49 Tpair/s, 0.88 of it (one CTA a tile, every thread through all atoms: 1.82); 96^3 x 8,192
+// 3.0 ms against 8.1, 64^3 x 4,000 0.50 against 2.0.
+template <int ZI, int XP, int UNR>
+__global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) fp64_pairs_kernel(const FwdParams p, const int vec_ok)
+{
+    constexpr int P = XP * ZI;
+    constexpr int R = 4 + ZI;  // doubles of a staged atom: x, y, q, (unused), dz of the planes
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    double* all = reinterpret_cast<double*>(smem_raw);
+    const int lane = threadIdx.x % 32;
+    const int warp = threadIdx.x / 32;
+    const int ranks = static_cast<int>(cluster_size());
+    double* rec = all + warp * (P > R ? P : R) * 32;
+    const int64_t column = static_cast<int64_t>(blockIdx.x / ranks) * 32 + lane;
+    const int yrow = static_cast<int>(column / p.columns);
+    const int x0 = static_cast<int>(column % p.columns) * XP;
+    const int z0 = p.z_base + static_cast<int>(blockIdx.y) * ZI;
+    double gx[XP], acc[XP][ZI];
+#pragma unroll
+    for (int k = 0; k < XP; ++k) {
+        gx[k] = static_cast<double>(fmaf(static_cast<float>(x0 + k), p.h, p.ox));
+#pragma unroll
+        for (int m = 0; m < ZI; ++m)
+            acc[k][m] = 0.0;
+    }
+    const double gy = static_cast<double>(fmaf(static_cast<float>(yrow), p.h, p.oy));
+    const int64_t shares = static_cast<int64_t>(ranks) * kRecordSplitWarps;
+    const int64_t w = static_cast<int64_t>(cluster_rank()) * kRecordSplitWarps + warp;
+    const int64_t end = p.n_atoms / shares * (w + 1) + p.n_atoms % shares * (w + 1) / shares;
+    int64_t b = p.n_atoms / shares * w + p.n_atoms % shares * w / shares;
+    float4 next = b + lane < end ? p.atoms[b + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (; b < end; b += 32) {
+        const int count = static_cast<int>(end - b < 32 ? end - b : 32);
+        __syncwarp();  // the previous atoms have been read
+        double2* r = reinterpret_cast<double2*>(rec + lane * R);
+        r[0] = make_double2(static_cast<double>(next.x), static_cast<double>(next.y));
+        r[1] = make_double2(static_cast<double>(next.w), 0.0);
+        const double az = static_cast<double>(next.z);
+#pragma unroll
+        for (int m = 0; m < ZI / 2; ++m)
+            r[2 + m] = make_double2(static_cast<double>(fmaf(static_cast<float>(z0 + 2 * m), p.h, p.oz)) - az,
+                                    static_cast<double>(fmaf(static_cast<float>(z0 + 2 * m + 1), p.h, p.oz)) - az);
+        __syncwarp();
+        if (b + 32 + lane < end)
+            next = p.atoms[b + 32 + lane];
+#pragma unroll UNR
+        for (int j = 0; j < count; ++j) {
+            const double2* a = reinterpret_cast<const double2*>(rec + j * R);
+            const double dy = gy - a[0].y;
+            const double dy2 = dy * dy;
+            const double q = a[1].x;
+            double dxy[XP];
+#pragma unroll
+            for (int k = 0; k < XP; ++k) {
+                const double dx = gx[k] - a[0].x;
+                dxy[k] = fma(dx, dx, dy2);
+            }
+#pragma unroll
+            for (int m = 0; m < ZI / 2; ++m) {
+                const double2 dz = a[2 + m];
+#pragma unroll
+                for (int k = 0; k < XP; ++k) {
+                    acc[k][2 * m] = pair_f64(dz.x, dxy[k], q, acc[k][2 * m]);
+                    acc[k][2 * m + 1] = pair_f64(dz.y, dxy[k], q, acc[k][2 * m + 1]);
+                }
+            }
+        }
+    }
+    __syncthreads();  // the warps' sums take the place of their atoms
+    double* sums = all + warp * P * 32 + lane;
+#pragma unroll
+    for (int m = 0; m < ZI; ++m)
+#pragma unroll
+        for (int k = 0; k < XP; ++k)
+            sums[(m * XP + k) * 32] = acc[k][m];
+    store_split_sums<XP, ZI, kRecordSplitWarps>(p, all, p.nz - z0 < ZI ? p.nz - z0 : ZI, x0, yrow, z0, vec_ok);
 }
 
 // Stores value i = (k * ZI + m) * nthreads + t of a tile's register blocks -- thread t's k-th x point,
@@ -1357,6 +1430,31 @@ struct VariantEntry {
     const void* occupancy_kernel;    // the kernel a persistent form sizes its grid by (else null)
 };
 
+// A launch of `kernel` on clusters of `ranks` CTAs along x (1: no cluster) of the split kernels' 256 threads.
+template <class... Args>
+cudaError_t launch_split_warps(void (*kernel)(Args...), const FwdLaunch& L, int ranks, cudaStream_t stream, Args... args)
+{
+    if (L.smem > 48u * 1024u) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(L.smem));
+        if (e != cudaSuccess)
+            return e;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = L.grid;
+    cfg.blockDim = dim3(32 * kRecordSplitWarps, 1, 1);
+    cfg.dynamicSmemBytes = L.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ranks);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ranks > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <int ZI, int XP, int UNR, int SRC, int SOA, int PREC, int SOFT, int MODE>
 cudaError_t launch_fwd(const FwdLaunch& L, cudaStream_t stream)
 {
@@ -1390,23 +1488,7 @@ cudaError_t launch_fwd(const FwdLaunch& L, cudaStream_t stream)
                 auto split = L.record_group == 8   ? record_split_kernel<ZI, XP, SOFT, 8>
                              : L.record_group == 4 ? record_split_kernel<ZI, XP, SOFT, 4>
                                                    : record_split_kernel<ZI, XP, SOFT, 2>;
-                const cudaError_t e = cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           static_cast<int>(L.smem));
-                if (e != cudaSuccess)
-                    return e;
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = L.grid;
-                cfg.blockDim = dim3(32 * kRecordSplitWarps, 1, 1);
-                cfg.dynamicSmemBytes = L.smem;
-                cfg.stream = stream;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = static_cast<unsigned>(L.record_ranks);
-                attr[0].val.clusterDim.y = 1;
-                attr[0].val.clusterDim.z = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = L.record_ranks > 1 ? 1 : 0;
-                return cudaLaunchKernelEx(&cfg, split, L.p, L.record_depth, L.vec_store);
+                return launch_split_warps(split, L, L.record_ranks, stream, L.p, L.record_depth, L.vec_store);
             }
         }
         if (L.smem > 48u * 1024u) {
@@ -1418,6 +1500,31 @@ cudaError_t launch_fwd(const FwdLaunch& L, cudaStream_t stream)
         kernel<<<L.grid, L.block, L.smem, stream>>>(L.p, L.vec_store);
         return cudaGetLastError();
     }
+}
+
+// The tile an FP64-pair variant runs: its own with up to 16 points a thread, 8 x 2 points for the wider ones,
+// whose sums alone take half of the 128 registers (8 x 4 points: 2.14 Tpair/s on 96^3 x 8,192, 8 x 2: 2.41).
+// A point's value does not depend on the tile.
+constexpr int fp64_zi(const int zi, const int xp) { return zi * xp > 16 ? 8 : zi; }
+constexpr int fp64_xp(const int zi, const int xp) { return zi * xp > 16 ? 2 : xp; }
+
+template <int ZI, int XP, int UNR>
+cudaError_t launch_fp64_pairs(const FwdLaunch& L, cudaStream_t stream)
+{
+    return launch_split_warps(fp64_pairs_kernel<fp64_zi(ZI, XP), fp64_xp(ZI, XP), UNR>, L, L.record_ranks, stream, L.p,
+                              L.vec_store);
+}
+
+template <int ZI, int XP, int UNR>
+void add_fp64_pairs_variant(std::vector<VariantEntry>& v)
+{
+    v.push_back(VariantEntry{VariantKey{ZI, XP, UNR, kSrcShared, 0, kPrecFp64Pairs, 0, kModeGrid3d, 0},
+                             &launch_fp64_pairs<ZI, XP, UNR>, 0, nullptr});
+}
+
+inline size_t fp64_pairs_smem_bytes(const int zi, const int xp)
+{
+    return static_cast<size_t>(kRecordSplitWarps) * 32 * sizeof(double) * (zi * xp > zi + 4 ? zi * xp : zi + 4);
 }
 
 template <int ZI, int XP, int UNR, int SRC, int SOA, int PREC, int SOFT, int MODE>

@@ -379,3 +379,35 @@ def test_record_tiles(ctx, n, block, nz):
             maps[prec, soft] = out
     for soft in (2, 12):
         assert torch.equal(maps[ktt_b200.PREC_FP64_MERGE, soft], maps[ktt_b200.PREC_FP64_MERGE_SHARED, soft])
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 33, 255, 257, 700])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (63, 2, 8), (65, 1, 9), (37, 41, 17), (130, 40, 21)])
+@pytest.mark.parametrize("shape", [(4, 1), (4, 4), (8, 4), (16, 1), (16, 2)])
+def test_fp64_pairs_shared_tiles(ctx, n, dims, shape):
+    """FP64 pairs, a tile's atoms split over warps and clusters: atom counts around the batches of 32 and
+    the warps' shares, tiles at the edges of the columns and planes.  Every point to the rounding of its
+    FP32 store (2^-24) plus the Newton step's 2^-40: 1.2e-7 with room for a sum's FP64 rounding; slabs
+    equal the map."""
+    import torch
+    rng = np.random.default_rng(n + dims[0])
+    a = np.empty((n, 4), dtype=np.float32)
+    a[:, :3] = rng.uniform(0.0, 20.0, (n, 3))
+    a[:, 3] = rng.uniform(0.1, 1.0, n)
+    h, origin = 0.5, (-1.0, 0.5, 2.0)
+    tune = ktt_b200.Tune(block_x=64, block_y=1, z_iterations=shape[0], x_points=shape[1],
+                         precision=ktt_b200.PREC_FP64_PAIRS)
+    atoms = _t(a) if n else torch.zeros((0, 4), device="cuda")
+    out = torch.full((dims[2], dims[1], dims[0]), float("nan"), device="cuda")
+    ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=out)
+    if n == 0:
+        assert torch.count_nonzero(out) == 0
+        return
+    ref = oracle.grid3d(a, h, dims, origin)
+    assert np.max(np.abs(_np(out) - ref) / np.abs(ref)) <= 1.2e-7
+    if dims[2] > 16:
+        assert torch.equal(ctx.forward_3d_slab(atoms, dims, h, 16, dims[2], origin, tune=tune), out[16:])
+    base = torch.linspace(-2, 2, out.numel(), device="cuda").reshape(out.shape)
+    acc = base.clone()
+    ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=acc, accumulate=True)
+    assert torch.equal(acc, base + out)
