@@ -1289,11 +1289,11 @@ __global__ void __launch_bounds__(kBalThreads, 1) balanced_split_kernel(const Fw
         // once this thread has given up, it no longer waits (its values are void anyway)
         if (!failed && !mbar_wait_bounded(&full[buf], (k / kStages) & 1u))
             failed = true;
-        // group grp's share of the stage: `per` atoms (a whole number of steps) from grp * per, the
-        // last step of a ragged share atom by atom
-        const int per = ((cnt + groups - 1) / groups + kBalAtomStep - 1) / kBalAtomStep * kBalAtomStep;
-        const int j_begin = grp * per;
-        const int j_count = cnt - j_begin < per ? cnt - j_begin : per;
+        // group grp's share of the stage, equal to one atom (whole steps of kBalAtomStep left one of the 32
+        // groups idle and the others up to 8 atoms more than their part: 72.4 us on 256 x 256 x 4,000, 70.3
+        // so); the last step of a ragged share atom by atom
+        const int j_begin = cnt * grp / groups;
+        const int j_count = cnt * (grp + 1) / groups - j_begin;
         if (j_count > 0) {
             const int j_full = j_begin + j_count / kBalAtomStep * kBalAtomStep;
             const int j_stop = j_begin + j_count;
