@@ -270,7 +270,9 @@ __device__ __forceinline__ float2 rsqrt_fma_x2(float2 x)
 // of (2k + 1) / 16; with NP >= 16 that share fits into one pattern, and pair p is soft where
 // (p + 1) (2k + 1) / 16 passes a whole number: 2k + 1 of every 16 pairs, spread evenly, so that a run of
 // MUFU pairs and a run of FMA-pipe pairs never wait for one another (5/16 of 16 pairs in a bare pair
-// loop: 6.30 Tpair/s spread, 6.05 side by side).  soft_phases is the number of stage phases of one whole
+// loop: 6.30 Tpair/s spread, 6.05 side by side).  In 2D the whole eighths of NP >= 8 pairs are spread in the
+// same way (a 1024 x 1024 slice x 20,000 atoms with 16 points a thread, 2/8: 3.68 ms, side by side 3.81); in
+// 3D they stay side by side, where the forms with FP64 sums lose 1.5 % by it.  soft_phases is the number of stage phases of one whole
 // pattern.
 constexpr int kSoftAlternate = 10;
 constexpr int soft_group(int np) { return np >= 8 ? 1 : 8 / np; }
@@ -295,11 +297,13 @@ __device__ __forceinline__ void with_phase(const int phase, F&& f)
     }
 }
 
-template <int SOFT, int NP, int PHASE>
+template <int SOFT, int NP, int PHASE, bool SPREAD>
 __device__ __forceinline__ constexpr bool pair_is_soft(int p)
 {
     if constexpr (SOFT >= kSoftAlternate && NP >= 16)
         return spread_soft(p, 2 * (SOFT - kSoftAlternate) + 1);
+    if constexpr (SPREAD && SOFT < kSoftAlternate && NP >= 8)
+        return spread_soft(p & 7, 2 * SOFT);
     constexpr int G = soft_group(NP);
     constexpr int base = SOFT >= kSoftAlternate ? SOFT - kSoftAlternate + PHASE / G : SOFT;
     return (NP >= 8 ? (p & 7) : (PHASE % G) * NP + p) < base;
@@ -343,7 +347,7 @@ __device__ __forceinline__ void pair_rows(const float (&pk)[XP], const float2 (&
     static_assert(ZA >= 1 && ZA <= ZH, "active pairs within the tile");
     if constexpr (K < XP) {
         if constexpr (I < ZA) {
-            constexpr bool soft = SOFT != 0 && pair_is_soft<SOFT, XP * ZH, PHASE>(K * ZH + P0 + I);
+            constexpr bool soft = SOFT != 0 && pair_is_soft<SOFT, XP * ZH, PHASE, !SQUARE_I>(K * ZH + P0 + I);
             constexpr bool half = HALF && I == ZA - 1;
             if constexpr (half) {
                 const float r2 = SQUARE_I ? fmaf(pi[I].x, pi[I].x, pk[K]) : fmaf(pk[K], pk[K], pi[I].x);
