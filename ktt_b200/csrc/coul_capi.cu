@@ -507,6 +507,23 @@ static int fp64_pairs_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tune* 
     return COUL_OK;
 }
 
+// FP32 sums of float4 atoms with 2 x 8 or 2 x 16 points a thread run the plain 3D kernel (2 x 16 points,
+// the tile's atoms split over eight warps and a cluster's CTAs) with the configuration's share of FMA-pipe
+// roots, whatever its block and unrolling, on maps of fewer than 64 of its tiles an SM: its tiles start at
+// multiples of their depth on the whole grid, so slabs still equal the map.  One CTA a tile leaves the
+// last tiles of such a map running alone.  Own tile and plain kernel, 2/8 share: 64 x 1 threads of 8 x 2 points,
+// 24^3 x 200 atoms 30 and 14 us, 64^3 x 2,000 167 and 114, 131 x 117 x 125 x 5,003 1,939 and 1,843, 128^3 x
+// 20,000 7.66 and 7.32 ms; 32 x 1 threads of 16 x 2 points, 128^3 x 20,000 9.15 and 7.32 ms.  Larger maps
+// have little left to gain (224^3 x 3,000 2 %) or lose (16 x 2 points, 5/16, 224^3 x 200: 393 and 421 us).
+static bool plain_tile(const coul_ctx* ctx, const VariantEntry* v, const coul_tune* t, int mode, const FwdParams& p, int nz)
+{
+    if (mode != kModeGrid3d || nz < 1 || v->key.split != 0 || v->key.soa != 0 || t->atom_source != COUL_ATOMS_SHARED_TMA ||
+        t->precision != COUL_PREC_FP32 || t->x_points != 2 || (t->z_iterations != 8 && t->z_iterations != 16))
+        return false;
+    const int64_t tiles_xy = ((p.nx + 1) / 2 * static_cast<int64_t>(p.ny) + 31) / 32;
+    return tiles_xy * ((nz + 15) / 16) < 64LL * ctx->sm_count;
+}
+
 // Launch one forward variant over a grid; shared by the 3D AoS/SoA and 2D entry points and by
 // the batched path's plain-launch baseline.
 int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz)
@@ -528,6 +545,10 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
     }
     if (gx > 2147483647LL || gy > 65535 || gz > 65535)
         return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
+    if (plain_tile(ctx, v, t, mode, prm, nz)) {
+        const int soft = t->rsqrt_soft;
+        return launch_plain_3d(ctx, prm, nz, soft >= kSoftAlternate ? 2 * (soft - kSoftAlternate) + 1 : 2 * soft);
+    }
     L.grid = dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
     if (v->key.split == 0 && linear_tiles(t->precision, t->z_iterations, mode)) {
         // linear x-y tiles where they are fewer than the block's rectangles

@@ -55,6 +55,9 @@ int validate_grid(const coul_grid* g);
 // nz: planes of the whole grid, by which a small 3D map's atoms are split over more CTAs (prm.z_base and
 // prm.nz bound the slab); 0: one warp runs through all atoms of a tile, as in the batched kernel.
 int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz);
+// The plain 3D kernel on planes [f.z_base, f.nz) of a map of nz planes, `soft` of 16 reciprocal square roots on
+// the FMA pipe (coul_plain.cu).
+int launch_plain_3d(coul_ctx* ctx, const FwdParams& f, int nz, int soft);
 int queue_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const coul_tune* t);
 int balanced_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const coul_tune* t);
 // Releases the device resources of the context's live batches and detaches them (coul_batched.cu);

@@ -2,7 +2,8 @@
 //
 // KTT leaves the choice of a kernel to its tuner; a caller without one (the PyTorch binding's plain
 // forward_3d / forward_2d) gets the kernels of this file, which suit every grid: a ligand's 40^3
-// points, a slice, a 256^3 map.  (One CTA per point tile of a fixed shape, as the configurable forms
+// points, a slice, a 256^3 map.  The 3D kernel also runs the configurations of 2 x 8 and 2 x 16 points a
+// thread with FP32 sums on maps of up to about 200^3 points (plain_tile).  (One CTA per point tile of a fixed shape, as the configurable forms
 // have it, leaves most SMs idle on the small ones: 33 CTAs for a 37 x 41 x 33 map.)
 //
 // A warp evaluates one point tile -- 32 columns of x points (columns numbered row by row over the
@@ -18,10 +19,10 @@
 //
 // Bound: the MUFU unit and the FMA pipe together (5/16 of the reciprocal square roots on the FMA
 // pipe in 3D, 2/8 in 2D).  On B200, against the default configuration's tile (128 x 4 x 16 points in
-// 3D, 128 x 16 in 2D, all roots on MUFU): 37 x 41 x 33 x 211 atoms 15 us a call against 87; 96^3 x 4,096 0.63 ms against 1.39;
-// 256^3 x 16,384 6.1 Tpair/s against 4.4; a 250 x 187 slice x 1,501 31 against 176 us (with the
-// conversion of its atoms).  What a thread's 32 points give
-// in 3D: 16 points (8 planes) reach 5.4.  100 registers and 16 warps an SM: 80 registers (24 warps)
+// 3D, 128 x 16 in 2D, all roots on MUFU): 37 x 41 x 33 x 211 atoms 15 us a call against 87; 96^3 x
+// 4,096 0.63 ms against 1.39; 256^3 x 16,384 6.1 Tpair/s against 4.4; a 250 x 187 slice x 1,501 30
+// against 176 us (with the conversion of its atoms).  What a thread's 32 points give in 3D: 16 points
+// (8 planes) reach 5.4.  100 registers and 16 warps an SM: 80 registers (24 warps)
 // spill a little and are 1 % slower, two atoms at a time are no faster.
 #include <cuda_runtime.h>
 
@@ -295,13 +296,8 @@ int launch_plain(coul_ctx* ctx, void (*kernel)(PlainParams), const PlainParams& 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = split > 1 ? 1 : 0;
-    int rc = ctx_begin_timing(ctx);
-    if (rc)
-        return rc;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
-    if (e != cudaSuccess)
-        return cuda_error(e, "forward launch");
-    return ctx_end_timing(ctx);
+    return e == cudaSuccess ? COUL_OK : cuda_error(e, "forward launch");
 }
 
 // CTAs that share a tile: twice as many while they leave half of the SMs without one, and while a
@@ -333,6 +329,37 @@ int check_call(const float* d_atoms, int64_t n_atoms, const float* d_out)
 
 }  // namespace
 
+int launch_plain_3d(coul_ctx* ctx, const FwdParams& f, int nz, int soft)
+{
+    void (*kernel)(PlainParams) = nullptr;
+    switch (soft) {
+    case 0: kernel = plain_3d_kernel<0>; break;
+    case 2: kernel = plain_3d_kernel<2>; break;
+    case 3: kernel = plain_3d_kernel<3>; break;
+    case 4: kernel = plain_3d_kernel<4>; break;
+    case 5: kernel = plain_3d_kernel<5>; break;
+    case 6: kernel = plain_3d_kernel<6>; break;
+    case 8: kernel = plain_3d_kernel<8>; break;
+    case 10: kernel = plain_3d_kernel<10>; break;
+    default: return set_error(COUL_ERR_UNSUPPORTED, "no kernel for this share of FMA-pipe roots");
+    }
+    PlainParams p{};
+    p.f = f;
+    p.columns = (f.nx + kPlainX - 1) / kPlainX;
+    const int64_t tiles_xy = (static_cast<int64_t>(p.columns) * f.ny + 31) / 32;
+    // The depth and the split follow from the whole grid, so that a slab's values are the map's.
+    p.vec_ok = f.nx % kPlainX == 0 && reinterpret_cast<uintptr_t>(f.out) % (kPlainX * sizeof(float)) == 0;
+    // Half the depth where full tiles would give a GPU of two CTAs an SM less than two rounds of them:
+    // 64^3 x 4,000 takes 203 us instead of 235.
+    const auto tiles_at = [&](int depth) { return tiles_xy * ((nz + depth - 1) / depth); };
+    p.depth = kPlainZ;
+    if (tiles_at(kPlainZ) < 4LL * ctx->sm_count && nz / (kPlainZ / 2) < 65535)
+        p.depth = kPlainZ / 2;
+    const int split = plain_split(ctx, tiles_at(p.depth), f.n_atoms, 5);
+    const int64_t tiles_z = (f.nz + p.depth - 1) / p.depth - f.z_base / p.depth;
+    return launch_plain(ctx, kernel, p, tiles_xy, tiles_z, split);
+}
+
 }  // namespace coul
 
 using namespace coul;
@@ -354,33 +381,22 @@ COUL_API int coul_forward_3d_plain(coul_ctx* ctx, const float* d_atoms, int64_t 
         return set_error(COUL_ERR_INVALID_ARGUMENT, "slab [z_begin, z_end) must be a non-empty range inside the grid");
     if ((rc = check_call(d_atoms, n_atoms, d_out)) || (rc = ctx_activate(ctx)))
         return rc;
-    PlainParams p{};
-    p.f.atoms = reinterpret_cast<const float4*>(d_atoms);
-    p.f.n_atoms = n_atoms;
-    p.f.nx = grid->nx;
-    p.f.ny = grid->ny;
-    p.f.nz = z_end;
-    p.f.z_base = z_begin;
-    p.f.h = grid->spacing;
-    p.f.ox = grid->origin[0];
-    p.f.oy = grid->origin[1];
-    p.f.oz = grid->origin[2];
-    p.f.out = d_out;
-    p.f.accumulate = accumulate ? 1 : 0;
-    p.columns = (grid->nx + kPlainX - 1) / kPlainX;
-    const int64_t tiles_xy = (static_cast<int64_t>(p.columns) * grid->ny + 31) / 32;
-    // The depth and the split follow from the whole grid, so that a slab's values are the map's.
-    p.vec_ok = grid->nx % kPlainX == 0 && reinterpret_cast<uintptr_t>(d_out) % (kPlainX * sizeof(float)) == 0;
-    // Half the depth where full tiles would give a GPU of two CTAs an SM less than two rounds of them:
-    // 64^3 x 4,000 takes 203 us instead of 235.
-    const auto tiles_at = [&](int depth) { return tiles_xy * ((grid->nz + depth - 1) / depth); };
-    p.depth = kPlainZ;
-    if (tiles_at(kPlainZ) < 4LL * ctx->sm_count && grid->nz / (kPlainZ / 2) < 65535)
-        p.depth = kPlainZ / 2;
-    const int split = plain_split(ctx, tiles_at(p.depth), n_atoms, 5);
-    const int64_t tiles_z = (z_end + p.depth - 1) / p.depth - z_begin / p.depth;
-    return launch_plain(ctx, n_atoms < kPlainSoftAtoms ? plain_3d_kernel<0> : plain_3d_kernel<5>, p, tiles_xy, tiles_z,
-                        split);
+    FwdParams f{};
+    f.atoms = reinterpret_cast<const float4*>(d_atoms);
+    f.n_atoms = n_atoms;
+    f.nx = grid->nx;
+    f.ny = grid->ny;
+    f.nz = z_end;
+    f.z_base = z_begin;
+    f.h = grid->spacing;
+    f.ox = grid->origin[0];
+    f.oy = grid->origin[1];
+    f.oz = grid->origin[2];
+    f.out = d_out;
+    f.accumulate = accumulate ? 1 : 0;
+    if ((rc = ctx_begin_timing(ctx)) || (rc = launch_plain_3d(ctx, f, grid->nz, n_atoms < kPlainSoftAtoms ? 0 : 5)))
+        return rc;
+    return ctx_end_timing(ctx);
 }
 
 COUL_API int coul_forward_2d_plain(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, float spacing, int nx, int ny,
@@ -407,7 +423,10 @@ COUL_API int coul_forward_2d_plain(coul_ctx* ctx, const float* d_atoms, int64_t 
     p.vec_ok = nx % kPlain2dX == 0 && aligned16(d_out);
     const int64_t tiles = (static_cast<int64_t>(p.columns) * ((ny + kPlain2dY - 1) / kPlain2dY) + 31) / 32;
     const int split = plain_split(ctx, tiles, n_atoms, 4);
-    return launch_plain(ctx, n_atoms < kPlainSoftAtoms ? plain_2d_kernel<0> : plain_2d_kernel<2>, p, tiles, 1, split);
+    if ((rc = ctx_begin_timing(ctx)) ||
+        (rc = launch_plain(ctx, n_atoms < kPlainSoftAtoms ? plain_2d_kernel<0> : plain_2d_kernel<2>, p, tiles, 1, split)))
+        return rc;
+    return ctx_end_timing(ctx);
 }
 
 }  // extern "C"

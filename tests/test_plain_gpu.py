@@ -85,3 +85,35 @@ def test_plain_call_keeps_the_refusals(ctx):
     for z0, z1 in ((-1, 4), (5, 5), (6, 3), (0, 9)):
         with pytest.raises(ktt_b200.CoulombError):
             ctx.forward_3d_slab(a, (8, 8, 8), 0.5, z0, z1, out=torch.empty((max(z1 - z0, 1), 8, 8), device="cuda"))
+
+
+@pytest.mark.parametrize("n", [0, 1, 33, 300, 700])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (63, 2, 8), (65, 1, 9), (37, 41, 17), (130, 40, 31)])
+@pytest.mark.parametrize("shape,soft", [((8, 2, 2), 2), ((8, 2, 1), 0), ((16, 2, 1), 12), ((8, 2, 1), 5)])
+def test_fp32_configurations_on_the_plain_kernel(ctx, n, dims, shape, soft):
+    """FP32 configurations of 8 x 2 and 16 x 2 points on a small map: a warp's sum of n / 8 terms, each
+    with the root's error (2.3e-7 rms, bias below 2^-21) and 2^-24 a step: below n / 8 * 2^-24 + 1e-6 of the
+    point's sum |q| / r.  Slabs at multiples of the configuration's depth equal the map; a sum adds to out."""
+    import torch
+    rng = np.random.default_rng(n + dims[0])
+    a = np.empty((n, 4), dtype=np.float32)
+    a[:, :3] = rng.uniform(0.0, 20.0, (n, 3))
+    a[:, 3] = rng.uniform(0.1, 1.0, n)
+    h, origin = 0.5, (-1.0, 0.5, 2.0)
+    tune = ktt_b200.Tune(block_x=64, block_y=1, z_iterations=shape[0], x_points=shape[1], unroll=shape[2],
+                         rsqrt_soft=soft)
+    atoms = torch.from_numpy(a).cuda() if n else torch.zeros((0, 4), device="cuda")
+    out = torch.full((dims[2], dims[1], dims[0]), float("nan"), device="cuda")
+    ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=out)
+    if n == 0:
+        assert torch.count_nonzero(out) == 0
+        return
+    ref = oracle.grid3d(a, h, dims, origin)
+    assert np.max(np.abs(out.cpu().numpy() - ref) / np.abs(ref)) <= n / 8 * 2.0**-24 + 1e-6
+    if dims[2] > shape[0]:
+        slab = ctx.forward_3d_slab(atoms, dims, h, shape[0], dims[2], origin, tune=tune)
+        assert torch.equal(slab, out[shape[0]:])
+    base = torch.linspace(-2, 2, out.numel(), device="cuda").reshape(out.shape)
+    acc = base.clone()
+    ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=acc, accumulate=True)
+    assert torch.equal(acc, base + out)
