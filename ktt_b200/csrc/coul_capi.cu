@@ -215,6 +215,8 @@ int ctx_activate(coul_ctx* ctx)
 
 int ctx_begin_timing(coul_ctx* ctx)
 {
+    if (ctx->timing_held)
+        return COUL_OK;
     cudaError_t e = cudaEventRecord(ctx->ev_start, ctx->stream);
     if (e != cudaSuccess)
         return cuda_error(e, "cudaEventRecord");
@@ -223,6 +225,8 @@ int ctx_begin_timing(coul_ctx* ctx)
 
 int ctx_end_timing(coul_ctx* ctx)
 {
+    if (ctx->timing_held)
+        return COUL_OK;
     cudaError_t e = cudaEventRecord(ctx->ev_stop, ctx->stream);
     if (e != cudaSuccess)
         return cuda_error(e, "cudaEventRecord");
@@ -722,6 +726,12 @@ COUL_API int coul_ctx_destroy(coul_ctx* ctx)
         cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop)
         cudaEventDestroy(ctx->ev_stop);
+    for (cudaEvent_t ev : ctx->slab_events)
+        if (ev)
+            cudaEventDestroy(ev);
+    for (cudaStream_t st : {ctx->second_stream, ctx->copy_stream})
+        if (st)
+            cudaStreamDestroy(st);
     if (ctx->own_stream)
         cudaStreamDestroy(ctx->own_stream);
     for (auto& f : ctx->cleanups)
@@ -1101,6 +1111,95 @@ COUL_API int coul_probe_bounded_wait(coul_ctx* ctx, int arrive, uint64_t budget_
     return coul_synchronize(ctx);
 }
 
+// Planes a slab of a host-buffer call (all of them: no slabs).  A slab is copied out while the next ones are
+// evaluated.  The call ends with the last slab's copy after the whole evaluation, or with all copies after
+// the first slab's evaluation, whichever is later; the depth that makes this least is taken, by the rates of
+// B200 (5.5 Tpair/s, FP64 pairs 2.4; a copy into pageable memory 30 us and 17 GB/s), where it saves 60 us.
+// In slabs and in one piece: 128^3 points x 8,192 atoms 3,146 and 3,505 us, 256^3 x 500 3.7 and 5.1 ms, but
+// 40 x 150 x 33 x 9,000 650 and 610 us, 128^3 x 250 in 16 planes 765 and 624 us.  The forms that split atoms
+// by the launch's own tiles, and those that go through the constant bank,
+// are not cut.
+static int slab_planes(const coul_grid* grid, int64_t n_atoms, const coul_tune* tune)
+{
+    if (tune && (tune->atom_split >= 2 || tune->atom_source != COUL_ATOMS_SHARED_TMA))
+        return grid->nz;
+    int step = 16;  // slabs at multiples of the tile's depth equal the map
+    while (tune && step % tune->z_iterations != 0)
+        step += 16;
+    const double points = static_cast<double>(grid->nx) * grid->ny;  // a plane's
+    const double evaluate = points * n_atoms / (tune && tune->precision == COUL_PREC_FP64_PAIRS ? 2.4e12 : 5.5e12);
+    const double copy = points * sizeof(float) / 17e9;
+    const double fixed = 30e-6;
+    int best = grid->nz;
+    double least = grid->nz * (evaluate + copy) - fixed;  // slabs have to save 60 us
+    for (int planes = (grid->nz / kHostSlabs / step + 1) * step; planes < grid->nz; planes += step) {
+        const int slabs = (grid->nz + planes - 1) / planes;
+        const int last = grid->nz - (slabs - 1) * planes;
+        const double time = std::max(grid->nz * evaluate + last * copy + fixed,
+                                     planes * evaluate + grid->nz * copy + slabs * fixed);
+        if (time < least) {
+            least = time;
+            best = planes;
+        }
+    }
+    return best;
+}
+
+// The map of a host-buffer call in slabs, on the context's stream and its second one in turn, so that a
+// slab's first tiles fill the SMs that the last tiles of the one before it leave; the copies on a third.
+static int host_slabs(coul_ctx* ctx, int64_t n_atoms, const coul_grid* grid, const coul_tune* tune, int planes, float* h_out)
+{
+    cudaError_t e = cudaSuccess;
+    for (cudaStream_t* st : {&ctx->second_stream, &ctx->copy_stream})
+        if (*st == nullptr && (e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking)) != cudaSuccess)
+            return cuda_error(e, "slab stream");
+    for (cudaEvent_t& ev : ctx->slab_events)
+        if (ev == nullptr && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+            return cuda_error(e, "slab event");
+    const cudaStream_t streams[2] = {ctx->stream, ctx->second_stream};
+    const size_t plane = static_cast<size_t>(grid->nx) * grid->ny;
+    int rc = ctx_begin_timing(ctx);
+    if (rc)
+        return rc;
+    // the atoms are there, and what this stream did before
+    if ((e = cudaEventRecord(ctx->slab_events[0], streams[0])) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(streams[1], ctx->slab_events[0], 0)) != cudaSuccess)
+        return cuda_error(e, "slab event");
+    ctx->timing_held = true;
+    int slabs = 0;
+    for (int z = 0; z < grid->nz && rc == COUL_OK; z += planes, ++slabs) {
+        const int z_end = std::min(z + planes, grid->nz);
+        float* out = ctx->d_out_cache + z * plane;
+        ctx->stream = streams[slabs % 2];
+        rc = tune ? coul_forward_3d_slab(ctx, ctx->d_atoms_cache, n_atoms, grid, z, z_end, tune, 0, out)
+                  : coul_forward_3d_plain(ctx, ctx->d_atoms_cache, n_atoms, grid, z, z_end, 0, out);
+        if (rc == COUL_OK && (e = cudaEventRecord(ctx->slab_events[slabs], ctx->stream)) != cudaSuccess)
+            rc = cuda_error(e, "slab event");
+    }
+    ctx->stream = streams[0];
+    ctx->timing_held = false;
+    // the timed region ends with the last slab of either stream
+    if (rc == COUL_OK && (e = cudaStreamWaitEvent(streams[0], ctx->slab_events[slabs - 1 - slabs % 2], 0)) != cudaSuccess)
+        rc = cuda_error(e, "slab event");
+    if (rc == COUL_OK)
+        rc = ctx_end_timing(ctx);
+    for (int i = 0; i < slabs && rc == COUL_OK; ++i) {
+        const size_t first = i * static_cast<size_t>(planes) * plane;
+        const size_t count = std::min(first + planes * plane, grid->nz * plane) - first;
+        if ((e = cudaStreamWaitEvent(ctx->copy_stream, ctx->slab_events[i], 0)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(h_out + first, ctx->d_out_cache + first, count * sizeof(float), cudaMemcpyDeviceToHost,
+                                 ctx->copy_stream)) != cudaSuccess)
+            rc = cuda_error(e, "map download");
+    }
+    // whatever happened, nothing is left behind on the other streams
+    for (cudaStream_t st : {ctx->second_stream, ctx->copy_stream}) {
+        e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess && rc == COUL_OK)
+            rc = cuda_error(e, "cudaStreamSynchronize");
+    }
+    return rc == COUL_OK ? coul_synchronize(ctx) : rc;
+}
+
 // tune NULL: the plain map
 static int forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms, const coul_grid* grid,
                            const coul_tune* tune, float* h_out)
@@ -1140,6 +1239,8 @@ static int forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms,
     if (abytes > 0 &&
         (e = cudaMemcpyAsync(ctx->d_atoms_cache, h_atoms, abytes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_error(e, "atom upload");
+    if (const int planes = slab_planes(grid, n_atoms, tune); planes < grid->nz)
+        return host_slabs(ctx, n_atoms, grid, tune, planes, h_out);
     rc = tune ? coul_forward_3d(ctx, ctx->d_atoms_cache, n_atoms, grid, tune, 0, ctx->d_out_cache)
               : coul_forward_3d_plain(ctx, ctx->d_atoms_cache, n_atoms, grid, 0, grid->nz, 0, ctx->d_out_cache);
     if (rc)

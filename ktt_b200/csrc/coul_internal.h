@@ -12,6 +12,8 @@
 
 struct coul_batch;
 
+constexpr int kHostSlabs = 16;  // slabs of a host-buffer call (at most)
+
 struct coul_ctx {
     int device = 0;
     void* user_context = nullptr;  // the caller's CUcontext (coul_ctx_create_on), else the primary context
@@ -20,6 +22,12 @@ struct coul_ctx {
     cudaEvent_t ev_start = nullptr; // bracket the most recent timed call
     cudaEvent_t ev_stop = nullptr;
     bool have_timing = false;
+    bool timing_held = false;       // a call of several launches records the events itself
+    // host-buffer calls in slabs (created by the first): every other slab's stream, the copies' stream, the
+    // slabs' ends
+    cudaStream_t second_stream = nullptr;
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t slab_events[kHostSlabs] = {};
     int* d_status = nullptr;  // device status word written by kernels whose bounded waits expire
     float* d_atoms_cache = nullptr;  // buffers of the host-pointer convenience calls
     size_t atoms_cap = 0;

@@ -411,3 +411,28 @@ def test_fp64_pairs_shared_tiles(ctx, n, dims, shape):
     acc = base.clone()
     ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=acc, accumulate=True)
     assert torch.equal(acc, base + out)
+
+
+@pytest.mark.parametrize("dims,n", [((130, 129, 33), 300), ((128, 128, 32), 5000), ((96, 90, 97), 1), ((90, 96, 100), 0),
+                                    ((257, 128, 47), 2000)])
+@pytest.mark.parametrize("fields", [None, dict(block_x=16, block_y=2, z_iterations=16, x_points=2, precision=4, rsqrt_soft=12),
+                                    dict(block_x=64, block_y=1, z_iterations=8, x_points=2, unroll=2, rsqrt_soft=2),
+                                    dict(block_x=64, block_y=1, z_iterations=32, x_points=1),
+                                    dict(block_x=64, block_y=1, z_iterations=8, x_points=4, precision=3),
+                                    dict(block_x=64, block_y=1, z_iterations=4, x_points=2, atom_source=1)])
+def test_host_buffer_call_in_slabs(ctx, dims, n, fields):
+    """Larger maps are evaluated and copied out in slabs of whole tiles: the host's map equals the device's bit
+    for bit, also with a last slab of one plane, and for forms that are not cut; the call is timed."""
+    rng = np.random.default_rng(n)
+    a = np.empty((n, 4), dtype=np.float32)
+    a[:, :3] = rng.uniform(0.0, 40.0, (n, 3))
+    a[:, 3] = rng.uniform(-1.0, 1.0, n)
+    tune = ktt_b200.Tune(**fields) if fields else None
+    import torch
+    atoms = _t(a) if n else torch.zeros((0, 4), device="cuda")
+    dev = ctx.forward_3d(atoms, dims, 0.5, (0.5, 0.25, -1.0), tune=tune)
+    ctx.synchronize()
+    for _ in range(2):
+        host = ctx.forward_3d_host(a, dims, 0.5, (0.5, 0.25, -1.0), tune=tune)
+        assert np.array_equal(host, _np(dev))
+        assert ctx.elapsed_ms() > 0.0
