@@ -486,9 +486,8 @@ static void record_split_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tun
                   static_cast<unsigned>((L.p.nz - L.p.z_base + depth - 1) / depth), 1);
 }
 
-// FP64 pairs: tiles of 32 linear columns, eight warps each, and as many CTAs of a
-// cluster as leave no SM without one while a warp keeps 8 atoms (from the whole grid's nz planes, so that
-// slabs equal the map).
+// FP64 pairs: tiles of 32 linear columns, eight warps each, and as many CTAs of a cluster as leave no SM
+// without one while a warp keeps 8 atoms (from the whole grid's nz planes, so that slabs equal the map).
 static int fp64_pairs_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tune* t, int nz)
 {
     const int zi = fp64_zi(t->z_iterations, t->x_points);
@@ -503,10 +502,7 @@ static int fp64_pairs_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tune* 
     if (tiles_xy * ranks > 2147483647LL)
         return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
     L.record_ranks = ranks;
-    const int64_t tiles_z = (L.p.nz - L.p.z_base + zi - 1) / zi;
-    if (tiles_z > 65535)
-        return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
-    L.grid = dim3(static_cast<unsigned>(tiles_xy * ranks), static_cast<unsigned>(tiles_z), 1);
+    L.grid = dim3(static_cast<unsigned>(tiles_xy * ranks), static_cast<unsigned>((L.p.nz - L.p.z_base + zi - 1) / zi), 1);
     L.smem = fp64_pairs_smem_bytes(zi, xp);
     return COUL_OK;
 }

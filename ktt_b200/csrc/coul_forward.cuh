@@ -1511,8 +1511,20 @@ constexpr int fp64_xp(const int zi, const int xp) { return zi * xp > 16 ? 2 : xp
 template <int ZI, int XP, int UNR>
 cudaError_t launch_fp64_pairs(const FwdLaunch& L, cudaStream_t stream)
 {
-    return launch_split_warps(fp64_pairs_kernel<fp64_zi(ZI, XP), fp64_xp(ZI, XP), UNR>, L, L.record_ranks, stream, L.p,
-                              L.vec_store);
+    // a grid holds 65,535 tiles along z; a configuration of deeper tiles than it runs may ask for more
+    constexpr unsigned kMost = 65535;
+    FwdLaunch part = L;
+    for (unsigned done = 0; done < L.grid.y; done += kMost) {
+        const int planes = static_cast<int>(done) * fp64_zi(ZI, XP);
+        part.grid.y = L.grid.y - done < kMost ? L.grid.y - done : kMost;
+        part.p.z_base = L.p.z_base + planes;
+        part.p.out = L.p.out + static_cast<int64_t>(planes) * L.p.ny * L.p.nx;
+        const cudaError_t e = launch_split_warps(fp64_pairs_kernel<fp64_zi(ZI, XP), fp64_xp(ZI, XP), UNR>, part,
+                                                 L.record_ranks, stream, part.p, L.vec_store);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 template <int ZI, int XP, int UNR>

@@ -3,8 +3,9 @@
 // KTT leaves the choice of a kernel to its tuner; a caller without one (the PyTorch binding's plain
 // forward_3d / forward_2d) gets the kernels of this file, which suit every grid: a ligand's 40^3
 // points, a slice, a 256^3 map.  The 3D kernel also runs the configurations of 2 x 8 and 2 x 16 points a
-// thread with FP32 sums on maps of up to about 200^3 points (plain_tile).  (One CTA per point tile of a fixed shape, as the configurable forms
-// have it, leaves most SMs idle on the small ones: 33 CTAs for a 37 x 41 x 33 map.)
+// thread with FP32 sums on maps of up to about 200^3 points (plain_tile).  (One CTA per point tile of a
+// fixed shape, as the configurable forms have it, leaves most SMs idle on the small ones: 33 CTAs for a
+// 37 x 41 x 33 map.)
 //
 // A warp evaluates one point tile -- 32 columns of x points (columns numbered row by row over the
 // plane, so only a row's end and the plane's end are padded) by 16 or 8 z points, or by 4 rows of a

@@ -436,3 +436,15 @@ def test_host_buffer_call_in_slabs(ctx, dims, n, fields):
         host = ctx.forward_3d_host(a, dims, 0.5, (0.5, 0.25, -1.0), tune=tune)
         assert np.array_equal(host, _np(dev))
         assert ctx.elapsed_ms() > 0.0
+
+
+def test_fp64_pairs_on_a_column_deeper_than_one_grid(ctx):
+    """A configuration of 16 planes a tile takes maps of up to 65,535 of them; the 8-plane tiles it runs then
+    need more than one grid's 65,535 along z.  To the FP32 store's rounding, 2^-24 and the Newton step's
+    2^-40: 1.2e-7."""
+    dims = (1, 1, 524_291)
+    a = np.array([[0.3, 0.2, 10.0, 1.0], [0.1, -0.4, 262_140.2, 0.5], [0.0, 0.1, 524_280.7, 0.25]], dtype=np.float32)
+    tune = ktt_b200.Tune(block_x=64, block_y=1, z_iterations=16, x_points=2, precision=ktt_b200.PREC_FP64_PAIRS)
+    out = _np(ctx.forward_3d(_t(a), dims, 1.0, tune=tune))
+    ref = oracle.grid3d(a, 1.0, dims)
+    assert np.max(np.abs(out - ref) / np.abs(ref)) <= 1.2e-7
