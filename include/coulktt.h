@@ -116,7 +116,12 @@ typedef struct coul_tune {
                          way the share is rsqrt_soft / 8.
                          10 + k (k = 0..7): a share of (2k + 1) / 16: with n >= 16 that many of every
                          16 pairs, spread evenly; with fewer, successive patterns alternate between k
-                         and k + 1 eighths */
+                         and k + 1 eighths.
+                         The FMA-pipe root holds for r^2 in 2^-100 .. 2^101.  Tiles of 2 x 16 points (float4
+                         atoms; FP32, FP64 merge), the small maps of 2 x 8 points on the plain kernel (FP32)
+                         and calls without a configuration send an atom outside that (on a grid point,
+                         or padding far away) through MUFU; the other forms with rsqrt_soft > 0 give
+                         NaN at the share's points for such atoms */
     int atom_split;   /* 0 or 1: one CTA per point tile; 2 or more: the atoms are split into that
                          many chunks per point tile, the partial sums of a tile added in chunk order
                          (for slices and small maps with too few tiles to fill the GPU; FP32,
@@ -276,7 +281,8 @@ COUL_API int coul_slice_atoms(coul_ctx* ctx, const float* d_xyzq, int64_t n_atom
 /*
  * The 3D map, or its slab [z_begin, z_end), and the 2D slice without a configuration: kernels that
  * suit every grid size (csrc/coul_plain.cu), FP32 pairs, sums at least as exact as those of
- * coul_tune_default().  Slabs put together equal the whole map bit for bit, whatever their
+ * coul_tune_default().  A point on an atom is +-inf and an atom of charge 0 adds 0 wherever it lies, infinity
+ * included.  Slabs put together equal the whole map bit for bit, whatever their
  * boundaries.  No counterpart in the reference, whose tuner picks a configuration for every launch.
  */
 COUL_API int coul_forward_3d_plain(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,

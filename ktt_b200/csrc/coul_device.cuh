@@ -250,6 +250,14 @@ __device__ __forceinline__ float2 rsqrt_fma_x2(float2 x)
     return __fmul2_rn(y, t);
 }
 
+// The FMA-pipe root is right for r^2 between 2^-100 and 2^101 (and for NaN).  Outside, where an FP32
+// coordinate difference squared underflows, overflows or is infinite, it is not what rsqrt gives: an atom on a
+// grid point (r^2 = 0) would come out NaN instead of q * inf, a charge-free atom put far away NaN instead of 0.
+// The kernels whose caller did not ask for that root therefore look at the atoms as they stage them and send a
+// batch that holds such an atom through MUFU.
+constexpr float kSoftNear = 0x1p-50f;  // a difference of at least this along one axis keeps r^2 above 2^-100
+constexpr float kSoftFar = 0x1p48f;    // coordinates below this on both sides keep r^2 below 2^101
+
 // ------------------------------------------------------------------------------------------
 // Pair blocks: one atom against a thread's register block of grid points.
 //

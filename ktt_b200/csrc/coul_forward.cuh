@@ -169,6 +169,25 @@ __device__ __forceinline__ void store_points(float* __restrict__ row, int x0, in
     }
 }
 
+// Whether an axis of the grid stays within the FMA-pipe root's range.
+__device__ __forceinline__ bool soft_axis(const int count, const float h, const float origin)
+{
+    return fabsf(origin) < kSoftFar && fabsf(fmaf(static_cast<float>(count), h, origin)) < kSoftFar;
+}
+
+// Whether every r^2 of an atom and a 3D tile is within that range, from the atom's place in x and y and its
+// smallest and largest |dz| to the tile's planes (the grid's own x and y are soft_axis').
+__device__ __forceinline__ bool soft_atom(const float4 a, const float dz_min, const float dz_max)
+{
+    return fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && dz_min >= kSoftNear && dz_max < kSoftFar;
+}
+
+__device__ __forceinline__ void dz_range(const float4 dz, float& dz_min, float& dz_max)
+{
+    dz_min = fminf(fminf(dz_min, fminf(fabsf(dz.x), fabsf(dz.y))), fminf(fabsf(dz.z), fabsf(dz.w)));
+    dz_max = fmaxf(fmaxf(dz_max, fmaxf(fabsf(dz.x), fabsf(dz.y))), fmaxf(fabsf(dz.z), fabsf(dz.w)));
+}
+
 // The first `count` records of a batch against a thread's columns: its first D planes, which are the
 // tile's from 2 * M0 on (the soft / MUFU choice goes by a plane's place among the tile's ZI).
 template <int XP, int ZI, int M0, int D, int SOFT>
@@ -210,6 +229,7 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
     constexpr int ZH = ZI / 2;
     static_assert(soft_phases(SOFT, XP * ZH) == 1 && kRecordMerge == 2 * kRecordAtoms, "one pattern, two batches a partial");
     float4* planes_z = rec + kRecordAtoms * record_floats(ZI) / 4;
+    const bool soft_grid = SOFT != 0 && soft_axis(p.nx, p.h, p.ox) && soft_axis(p.ny, p.h, p.oy);
     __syncwarp();  // a persistent kernel's previous tile has been read
     for (int m = lane; m < ZI; m += lanes)
         reinterpret_cast<float*>(planes_z)[m] = fmaf(static_cast<float>(z0 + m), p.h, p.oz);
@@ -219,20 +239,28 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
     for (int64_t b = a0; b < a1; b += kRecordAtoms) {
         const int count = static_cast<int>(a1 - b < kRecordAtoms ? a1 - b : kRecordAtoms);
         __syncwarp();  // the previous records have been read
+        bool inside = soft_grid;
         for (int j = lane; j < count; j += lanes) {
             const float4 a = j == lane ? next : p.atoms[b + j];
             float4* r = rec + j * (record_floats(ZI) / 4);
             r[0] = make_float4(a.x, a.y, a.w, a.w * kSoftRsqrtScale);
+            float dz_min = kSoftFar, dz_max = 0.0f;
 #pragma unroll
             for (int m = 0; m < ZI / 4; ++m) {
                 const float4 z = planes_z[m];
-                r[1 + m] = make_float4(z.x - a.z, z.y - a.z, z.z - a.z, z.w - a.z);
+                const float4 dz = make_float4(z.x - a.z, z.y - a.z, z.z - a.z, z.w - a.z);
+                r[1 + m] = dz;
+                dz_range(dz, dz_min, dz_max);
             }
+            inside = inside && soft_atom(a, dz_min, dz_max);
         }
+        const bool soft = SOFT == 0 || __all_sync(0xffffffffu >> (32 - lanes), inside);
         __syncwarp();
         if (lane < kRecordAtoms && b + kRecordAtoms + lane < a1)
             next = p.atoms[b + kRecordAtoms + lane];
-        if (HALVES && sub != 0)
+        if (!soft)
+            record_batch<XP, ZI, 0, ZI, 0>(rec, count, gx, gy, acc);  // planes past the tile's end are not stored
+        else if (HALVES && sub != 0)
             with_phase<ZH / 2>(pairs - 1, [&](auto q) {
                 record_batch<XP, ZI, ZH / 2, 2 * (decltype(q)::value + 1), SOFT>(rec, count, gx, gy, acc);
             });

@@ -186,25 +186,37 @@ __global__ void __launch_bounds__(kPlainThreads, 2) plain_3d_kernel(const PlainP
 
     int64_t b, end;
     warp_atoms(p.f.n_atoms, ranks, b, end);
+    const bool soft_grid = SOFT != 0 && soft_axis(p.f.nx, p.f.h, p.f.ox) && soft_axis(p.f.ny, p.f.h, p.f.oy);
     float4* rec = reinterpret_cast<float4*>(s_warp[warp]);
     float4 a = b + lane < end ? p.f.atoms[b + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (; b < end; b += 32) {
         const int cnt = static_cast<int>(end - b < 32 ? end - b : 32);
         __syncwarp();  // the previous records have been read
         rec[lane * (kPlainRecord / 4)] = make_float4(a.x, a.y, a.w, a.w * kSoftRsqrtScale);
+        float dz_min = kSoftFar, dz_max = 0.0f;  // over the planes of the tile, whichever of them a slab asks for
 #pragma unroll
         for (int m = 0; m < kPlainZ / 4; ++m) {
             const float4 g = s_gz[m];
-            rec[lane * (kPlainRecord / 4) + 1 + m] = make_float4(g.x - a.z, g.y - a.z, g.z - a.z, g.w - a.z);
+            const float4 dz = make_float4(g.x - a.z, g.y - a.z, g.z - a.z, g.w - a.z);
+            rec[lane * (kPlainRecord / 4) + 1 + m] = dz;
+            if (4 * m < p.depth)
+                dz_range(dz, dz_min, dz_max);
         }
+        const bool soft = SOFT != 0 && __all_sync(0xffffffffu, lane >= cnt || (soft_grid && soft_atom(a, dz_min, dz_max)));
         __syncwarp();
         if (b + 32 + lane < end)
             a = p.f.atoms[b + 32 + lane];
         // a tile that overhangs the grid by half or more evaluates its first half
-        if (planes <= kPlainZ / 2)
-            plain_batch<SOFT, kPlainZ / 2>(rec, cnt, gx, gy, acc);
-        else
+        if (planes <= kPlainZ / 2) {
+            if (soft)
+                plain_batch<SOFT, kPlainZ / 2>(rec, cnt, gx, gy, acc);
+            else
+                plain_batch<0, kPlainZ / 2>(rec, cnt, gx, gy, acc);
+        } else if (soft) {
             plain_batch<SOFT, kPlainZ>(rec, cnt, gx, gy, acc);
+        } else {
+            plain_batch<0, kPlainZ>(rec, cnt, gx, gy, acc);
+        }
     }
     __syncwarp();
 #pragma unroll
@@ -253,18 +265,29 @@ __global__ void __launch_bounds__(kPlainThreads, 4) plain_2d_kernel(const PlainP
 
     int64_t b, end;
     warp_atoms(p.f.n_atoms, ranks, b, end);
+    const bool soft_grid = SOFT != 0 && soft_axis(p.f.nx, p.f.h, p.f.ox) && soft_axis(p.f.ny, p.f.h, p.f.oy);
     float4* rec = reinterpret_cast<float4*>(s_warp[warp]);
     float4 a = b + lane < end ? p.f.atoms[b + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (; b < end; b += 32) {
         const int cnt = static_cast<int>(end - b < 32 ? end - b : 32);
         __syncwarp();
         rec[lane] = a;
+        // an atom's .z is its dz^2 to the slice
+        const bool inside = fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && a.z >= kSoftNear * kSoftNear &&
+                            a.z < kSoftFar * kSoftFar;
+        const bool soft = SOFT != 0 && __all_sync(0xffffffffu, lane >= cnt || (soft_grid && inside));
         __syncwarp();
         if (b + 32 + lane < end)
             a = p.f.atoms[b + 32 + lane];
+        if (soft) {
 #pragma unroll 2
-        for (int j = 0; j < cnt; ++j)
-            pair_block_2d<kPlain2dX, YH, YH, SOFT, 0, false>(gx, gy, rec[j], acc);
+            for (int j = 0; j < cnt; ++j)
+                pair_block_2d<kPlain2dX, YH, YH, SOFT, 0, false>(gx, gy, rec[j], acc);
+        } else {
+#pragma unroll 2
+            for (int j = 0; j < cnt; ++j)
+                pair_block_2d<kPlain2dX, YH, YH, 0, 0, false>(gx, gy, rec[j], acc);
+        }
     }
     __syncwarp();
 #pragma unroll

@@ -117,3 +117,83 @@ def test_fp32_configurations_on_the_plain_kernel(ctx, n, dims, shape, soft):
     acc = base.clone()
     ctx.forward_3d(atoms, dims, h, origin, tune=tune, out=acc, accumulate=True)
     assert torch.equal(acc, base + out)
+
+
+def _places(n, seed):
+    """n atoms of which 32 lie on grid points (spacing 0.5, origin 0), one for every place in a tile of 2 x 16
+    points a thread, and 8 without charge lie beyond FP32's r^2: what pads a molecule."""
+    a = _atoms(n, seed)
+    rng = np.random.default_rng(seed + 1)
+    pick = rng.permutation(n)
+    for i in range(32):
+        a[pick[i], :3] = 0.5 * np.array([i, i % 7, (5 * i + i // 16) % 16])
+    far = np.array([[1e20, 0, 0], [0, -1e20, 0], [0, 0, 1e20], [np.inf, 1, 2], [1, -np.inf, 2], [1, 2, np.inf],
+                    [3e38, 3e38, 3e38], [-np.inf, np.inf, -np.inf]], dtype=np.float32)
+    a[pick[32:40], :3] = far
+    a[pick[32:40], 3] = 0.0
+    return a, pick[:32]
+
+
+def _check_places(out, a, hits, exact):
+    """`out` (last axis x, spacing 0.5) is q * inf on the atoms `hits` and the exact map elsewhere."""
+    at = np.round(a[hits, :3] * 2).astype(int)
+    mask = np.zeros(out.shape, dtype=bool)
+    for (x, y, z), q in zip(at, a[hits, 3]):
+        index = (z, y, x) if out.ndim == 3 else (y, x)
+        assert out[index] == np.copysign(np.inf, q), (x, y, z)
+        mask[index] = True
+    assert np.all(np.isfinite(out[~mask]))
+    ref = exact[~mask]
+    assert np.linalg.norm(out[~mask] - ref) <= TOL * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [100, 511, 512, 2049])
+@pytest.mark.parametrize("dims", [(40, 9, 16), (37, 13, 41), (96, 64, 48)])
+@pytest.mark.parametrize("fields", [None, dict(z_iterations=8, x_points=2, unroll=2, rsqrt_soft=2),
+                                    dict(z_iterations=16, x_points=2, rsqrt_soft=12, precision=4)])
+def test_atoms_on_grid_points_and_beyond_range(ctx, dims, n, fields):
+    """A point on an atom is +-inf and an atom without charge adds nothing wherever it lies, also where a pair's
+    root runs on the FMA pipe, whose arithmetic holds for r^2 in 2^-100 .. 2^101 only."""
+    import torch
+    a, hits = _places(n, n)
+    tune = ktt_b200.Tune(block_x=16, block_y=2, **fields) if fields else None
+    out = ctx.forward_3d(_cuda(a), dims, 0.5, tune=tune)
+    with np.errstate(divide="ignore"):
+        ref = oracle.grid3d(np.delete(a, np.where(a[:, 3] == 0)[0], axis=0), 0.5, dims)
+    _check_places(out.cpu().numpy(), a, hits, ref)
+    if dims[2] > 16:
+        assert torch.equal(ctx.forward_3d_slab(_cuda(a), dims, 0.5, 16, dims[2], tune=tune), out[16:])
+    if fields and n == 512:
+        batch = ktt_b200.Batch(ctx, [(_cuda(a), dims, 0.5, (0.0, 0.0, 0.0))],
+                               ktt_b200.Tune(block_x=7, block_y=3, z_iterations=16, x_points=2, rsqrt_soft=12, precision=4))
+        batch.run()
+        ctx.synchronize()
+        _check_places(batch.outputs[0].cpu().numpy(), a, hits, ref)
+        batch.close()
+
+
+@pytest.mark.parametrize("n", [100, 511, 512, 2049])
+def test_atoms_on_slice_points_and_beyond_range(ctx, n):
+    a, hits = _places(n, n)
+    flat = a.copy()
+    with np.errstate(over="ignore"):
+        flat[:, 2] = (np.float32(7.3) - a[:, 2]) ** 2
+    flat[hits, 2] = 0.0
+    flat[hits, 1] = 0.5 * (np.arange(32) % 7)
+    out = ctx.forward_2d(_cuda(flat), 0.5, 61, 30).cpu().numpy()
+    with np.errstate(divide="ignore"):
+        ref = oracle.slice2d(np.delete(flat, np.where(flat[:, 3] == 0)[0], axis=0), 0.5, 61, 30)
+    _check_places(out, flat, hits, ref)
+
+
+@pytest.mark.parametrize("n", [600, 3000])
+def test_atoms_closer_than_the_range_of_the_root(ctx, n):
+    """Distances whose square is small, subnormal or zero in FP32, at the origin's point: MUFU's value, which
+    flushes a subnormal r^2 to zero.  One charge near the point dominates it by 1e10 and more."""
+    a = _atoms(n, seed=n) + np.array([1, 1, 1, 0], dtype=np.float32)
+    for k in range(32):  # the point's place in its tile
+        origin = (-0.5 * (k % 2), 0.0, -0.5 * (k // 2))
+        for r, want in ((1e-14, 1e14), (3e-16, 1 / 3e-16), (1e-18, 1e18), (1e-20, np.inf), (1e-30, np.inf)):
+            a[7] = ((0.0, 0.0, r, 1.0), (r, 0.0, 0.0, 1.0))[k % 2]
+            got = ctx.forward_3d(_cuda(a), (96, 64, 32), 0.5, origin)[k // 2, 0, k % 2].item()
+            assert got == want or abs(got / want - 1) <= 1e-6, (k, r)
