@@ -117,7 +117,9 @@ typedef struct coul_tune {
                          10 + k (k = 0..7): a share of (2k + 1) / 16: with n >= 16 that many of every
                          16 pairs, spread evenly; with fewer, successive patterns alternate between k
                          and k + 1 eighths.
-                         The FMA-pipe root holds for r^2 in 2^-100 .. 2^101.  Tiles of 2 x 16 points (float4
+                         The FMA-pipe root is good to 4.6e-7 (MUFU: 1.3e-7); tiles of 2 x 16 points with FP64
+                         merge, and calls without a configuration, take a longer one, good to 1.1e-7.
+                         It holds for r^2 in 2^-100 .. 2^101.  Tiles of 2 x 16 points (float4
                          atoms; FP32, FP64 merge), the small maps of 2 x 8 points on the plain kernel (FP32)
                          and calls without a configuration send an atom outside that (on a grid point,
                          or padding far away) through MUFU; the other forms with rsqrt_soft > 0 give
@@ -280,8 +282,8 @@ COUL_API int coul_slice_atoms(coul_ctx* ctx, const float* d_xyzq, int64_t n_atom
                               float* d_xy_dz2_q);
 /*
  * The 3D map, or its slab [z_begin, z_end), and the 2D slice without a configuration: kernels that
- * suit every grid size (csrc/coul_plain.cu), FP32 pairs, sums at least as exact as those of
- * coul_tune_default().  A point on an atom is +-inf and an atom of charge 0 adds 0 wherever it lies, infinity
+ * suit every grid size (csrc/coul_plain.cu), FP32 pairs, roots (1.3e-7) and sums at least as exact as those
+ * of coul_tune_default().  A point on an atom is +-inf and an atom of charge 0 adds 0 wherever it lies, infinity
  * included.  Slabs put together equal the whole map bit for bit, whatever their
  * boundaries.  No counterpart in the reference, whose tuner picks a configuration for every launch.
  */

@@ -250,10 +250,42 @@ __device__ __forceinline__ float2 rsqrt_fma_x2(float2 x)
     return __fmul2_rn(y, t);
 }
 
-// The FMA-pipe root is right for r^2 between 2^-100 and 2^101 (and for NaN).  Outside, where an FP32
-// coordinate difference squared underflows, overflows or is infinite, it is not what rsqrt gives: an atom on a
+// The same at MUFU's precision, for the forms whose caller did not choose the root above: one step of fourth
+// order, 1/sqrt(x) = y (1 + e)^(-1/2) with e = x y^2 - 1, |e| < 0.069 for this constant, and (1 + e)^(-1/2) - 1 by
+// its minimax polynomial e (c1 + c2 e + c3 e^2 + c4 e^3) (residual 2.3e-8).  Adding the small correction to y
+// leaves one full rounding: relative error in [-1.08e-7, 1.10e-7], rms 3.2e-8, over all normal inputs (rsqrt.approx:
+// 2^-22.9 = 1.28e-7), and no scale.  2 integer + 7 FP32 instructions; all packed: with the polynomial's steps as
+// scalar FMAs with immediates 256^3 x 65,536 takes 199 ms, by pairs of terms 202, so 193.1.  Derivation and exhaustive
+// check: ktt_b200/soft_rsqrt.py.
+constexpr uint32_t kFullRsqrtMagic = 0x5f375000u;
+constexpr float kFullRsqrtC1 = -0.49999833f;
+constexpr float kFullRsqrtC2 = 0.3749989f;
+constexpr float kFullRsqrtC3 = -0.31393645f;
+constexpr float kFullRsqrtC4 = 0.27455508f;
+
+__device__ __forceinline__ float rsqrt_full(float x)
+{
+    const float y = __uint_as_float(kFullRsqrtMagic - (__float_as_uint(x) >> 1));
+    const float e = fmaf(x, y * y, -1.0f);
+    const float c = fmaf(fmaf(fmaf(e, kFullRsqrtC4, kFullRsqrtC3), e, kFullRsqrtC2), e, kFullRsqrtC1);
+    return fmaf(y, e * c, y);
+}
+
+__device__ __forceinline__ float2 rsqrt_full_x2(float2 x)
+{
+    const float2 y = make_float2(__uint_as_float(kFullRsqrtMagic - (__float_as_uint(x.x) >> 1)),
+                                 __uint_as_float(kFullRsqrtMagic - (__float_as_uint(x.y) >> 1)));
+    const float2 e = __ffma2_rn(x, __fmul2_rn(y, y), splat(-1.0f));
+    float2 c = __ffma2_rn(e, splat(kFullRsqrtC4), splat(kFullRsqrtC3));
+    c = __ffma2_rn(c, e, splat(kFullRsqrtC2));
+    c = __ffma2_rn(c, e, splat(kFullRsqrtC1));
+    return __ffma2_rn(y, __fmul2_rn(e, c), y);
+}
+
+// The FMA-pipe roots are right for r^2 between 2^-100 and 2^101 (and for NaN).  Outside, where an FP32
+// coordinate difference squared underflows, overflows or is infinite, they are not what rsqrt gives: an atom on a
 // grid point (r^2 = 0) would come out NaN instead of q * inf, a charge-free atom put far away NaN instead of 0.
-// The kernels whose caller did not ask for that root therefore look at the atoms as they stage them and send a
+// The kernels whose caller did not ask for those roots therefore look at the atoms as they stage them and send a
 // batch that holds such an atom through MUFU.
 constexpr float kSoftNear = 0x1p-50f;  // a difference of at least this along one axis keeps r^2 above 2^-100
 constexpr float kSoftFar = 0x1p48f;    // coordinates below this on both sides keep r^2 below 2^101
@@ -283,10 +315,14 @@ constexpr float kSoftFar = 0x1p48f;    // coordinates below this on both sides k
 // 3D they stay side by side, where the forms with FP64 sums lose 1.5 % by it.  soft_phases is the number of stage phases of one whole
 // pattern.
 constexpr int kSoftAlternate = 10;
+// SOFT = share + kSoftFull: the share's pairs take rsqrt_full, and the charge as it is
+constexpr int kSoftFull = 64;
+constexpr int soft_share(int soft) { return soft % kSoftFull; }
+constexpr float soft_scale(int soft) { return soft >= kSoftFull ? 1.0f : kSoftRsqrtScale; }
 constexpr int soft_group(int np) { return np >= 8 ? 1 : 8 / np; }
 constexpr int soft_phases(int soft, int np)
 {
-    return soft == 0 || np >= 16 ? 1 : (soft >= kSoftAlternate ? 2 : 1) * soft_group(np);
+    return soft == 0 || np >= 16 ? 1 : (soft_share(soft) >= kSoftAlternate ? 2 : 1) * soft_group(np);
 }
 constexpr bool spread_soft(int p, int sixteenths) { return (p + 1) * sixteenths / 16 != p * sixteenths / 16; }
 
@@ -322,20 +358,24 @@ __device__ __forceinline__ float2 rsqrt_mufu_x2(float2 r2)
     return make_float2(rsqrt_mufu(r2.x), rsqrt_mufu(r2.y));
 }
 
-// One lane pair: acc += q / sqrt(r2) lane-wise, the rsqrt on the FMA pipe when SOFT_PAIR (the charge
-// then comes pre-scaled by kSoftRsqrtScale in qs2).  HALF_PAIR: only the .x lane holds a point (an
+// One lane pair: acc += q / sqrt(r2) lane-wise, the rsqrt on the FMA pipe when SOFT_PAIR: rsqrt_full when FULL,
+// else rsqrt_fma (the charge then comes pre-scaled by kSoftRsqrtScale in qs2).  HALF_PAIR: only the .x lane holds a point (an
 // odd number of points along the blocked axis); it is evaluated alone, so no rsqrt is spent on a
 // point that is never stored.
-template <bool SOFT_PAIR, bool HALF_PAIR>
+template <bool SOFT_PAIR, bool FULL, bool HALF_PAIR>
 __device__ __forceinline__ void pair_update(float2 r2, float2 q2, float2 qs2, float2& acc)
 {
     if constexpr (HALF_PAIR) {
-        if constexpr (SOFT_PAIR)
+        if constexpr (SOFT_PAIR && FULL)
+            acc.x = fmaf(q2.x, rsqrt_full(r2.x), acc.x);
+        else if constexpr (SOFT_PAIR)
             acc.x = fmaf(qs2.x, rsqrt_fma(r2.x), acc.x);
         else
             acc.x = fmaf(q2.x, rsqrt_mufu(r2.x), acc.x);
     } else {
-        if constexpr (SOFT_PAIR)
+        if constexpr (SOFT_PAIR && FULL)
+            acc = __ffma2_rn(q2, rsqrt_full_x2(r2), acc);
+        else if constexpr (SOFT_PAIR)
             acc = __ffma2_rn(qs2, rsqrt_fma_x2(r2), acc);
         else
             acc = __ffma2_rn(q2, rsqrt_mufu_x2(r2), acc);
@@ -355,15 +395,15 @@ __device__ __forceinline__ void pair_rows(const float (&pk)[XP], const float2 (&
     static_assert(ZA >= 1 && ZA <= ZH, "active pairs within the tile");
     if constexpr (K < XP) {
         if constexpr (I < ZA) {
-            constexpr bool soft = SOFT != 0 && pair_is_soft<SOFT, XP * ZH, PHASE, !SQUARE_I>(K * ZH + P0 + I);
+            constexpr bool soft = SOFT != 0 && pair_is_soft<soft_share(SOFT), XP * ZH, PHASE, !SQUARE_I>(K * ZH + P0 + I);
             constexpr bool half = HALF && I == ZA - 1;
             if constexpr (half) {
                 const float r2 = SQUARE_I ? fmaf(pi[I].x, pi[I].x, pk[K]) : fmaf(pk[K], pk[K], pi[I].x);
-                pair_update<soft, true>(make_float2(r2, 0.0f), q2, qs2, acc[K][I]);
+                pair_update<soft, SOFT >= kSoftFull, true>(make_float2(r2, 0.0f), q2, qs2, acc[K][I]);
             } else {
                 const float2 r2 = SQUARE_I ? __ffma2_rn(pi[I], pi[I], splat(pk[K]))
                                            : __ffma2_rn(splat(pk[K]), splat(pk[K]), pi[I]);
-                pair_update<soft, false>(r2, q2, qs2, acc[K][I]);
+                pair_update<soft, SOFT >= kSoftFull, false>(r2, q2, qs2, acc[K][I]);
             }
             pair_rows<SQUARE_I, XP, ZH, ZA, SOFT, PHASE, HALF, P0, K, I + 1>(pk, pi, q2, qs2, acc);
         } else {

@@ -227,7 +227,7 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
                                              const float (&gx)[XP], const float gy, float2 (&acc)[XP][ZI / 2], Merge&& merge)
 {
     constexpr int ZH = ZI / 2;
-    static_assert(soft_phases(SOFT, XP * ZH) == 1 && kRecordMerge == 2 * kRecordAtoms, "one pattern, two batches a partial");
+    static_assert(soft_phases(SOFT, XP * ZH) == 1 && kRecordMerge % kRecordAtoms == 0, "one pattern, whole batches a partial");
     float4* planes_z = rec + kRecordAtoms * record_floats(ZI) / 4;
     const bool soft_grid = SOFT != 0 && soft_axis(p.nx, p.h, p.ox) && soft_axis(p.ny, p.h, p.oy);
     __syncwarp();  // a persistent kernel's previous tile has been read
@@ -235,7 +235,7 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
         reinterpret_cast<float*>(planes_z)[m] = fmaf(static_cast<float>(z0 + m), p.h, p.oz);
     const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float4 next = lane < kRecordAtoms && a0 + lane < a1 ? p.atoms[a0 + lane] : none;
-    bool odd = false;
+    int batches = 0;  // of the partial so far; a flag that is flipped instead makes the pair loop 1.7 % slower
     for (int64_t b = a0; b < a1; b += kRecordAtoms) {
         const int count = static_cast<int>(a1 - b < kRecordAtoms ? a1 - b : kRecordAtoms);
         __syncwarp();  // the previous records have been read
@@ -270,20 +270,29 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
             with_phase<ZH - 1>(pairs - 1, [&](auto q) {
                 record_batch<XP, ZI, 0, 2 * (decltype(q)::value + 1), SOFT>(rec, count, gx, gy, acc);
             });
-        if (odd)
+        if (++batches == kRecordMerge / kRecordAtoms) {
             merge();
-        odd = !odd;
+            batches = 0;
+        }
     }
-    if (odd)
+    if (batches != 0)
         merge();
+}
+
+// The FMA-pipe roots of the FP64-merge record tiles are the full ones: five sixteenths of rsqrt_fma's, where 8 x 2
+// points had four, made the gradient of a fit 12 % (charges) and 5 % (positions) less exact (mean of 12 drawn fits).
+// Errors against 64 bits with 8 x 2 points and 4/16, 2 x 16 and 5/16 of rsqrt_fma, the same of rsqrt_full: 128^3 x
+// 8,192 2.58e-7, 2.49e-7, 1.77e-7; the fits' gradients 1, 1.12, 0.41 and 1, 1.05, 0.65; 12 to 32 molecules
+// 2.3e-7, 2.3e-7, 1.7e-7; 256^3 x 65,536 in 195.9, 186.4, 193.1 ms.
+constexpr int record_soft(const int prec, const int soft)
+{
+    return prec == kPrecFp32 || soft == 0 ? soft : soft + kSoftFull;
 }
 
 // tile_accumulate for record tiles: a warp needs no other.  On 256^3 x 65,536 with 5/16 of the roots on
 // the FMA pipe: FP32 sums 180.1 ms = 6.10 Tpair/s (8 x 2 points through the TMA ring, 2/8: 191.8 ms), FP64
-// merge 187.4 ms = 5.87 Tpair/s (195.9).  An FP32 partial of 48 atoms, not kMergeAtoms: the shorter sums
-// take back what the larger share of FMA-pipe roots adds to the error (64-bit error of a 128^3 map
-// 2.49e-7; 8 x 2 points with 64 atoms and 2/8: 2.58e-7; 96 atoms 2 % faster but 3.00e-7, 32 atoms 2 %
-// slower, 6/16 with 48 1 % faster but 2.61e-7).
+// merge 193.1 ms = 5.69 Tpair/s (195.9; atoms split, record_split_kernel).  An FP32 partial of 48 atoms, not
+// kMergeAtoms: 72 and 96 are no faster (194.4, 193.4 ms) and less exact (128^3 x 8,192 1.77e-7, 2.03e-7, 2.44e-7).
 template <int ZI, int XP, int PREC, int SOFT>
 __device__ __forceinline__ void record_accumulate(const FwdParams& p, const int x0, const int yrow, const int z0,
                                                   unsigned char* smem, float (&val)[XP][ZI])
@@ -320,7 +329,8 @@ __device__ __forceinline__ void record_accumulate(const FwdParams& p, const int 
     clear();
     // a tile that overhangs the grid evaluates its planes inside it, in pairs of planes
     const int pairs = p.nz - z0 < ZI ? (p.nz - z0 + 1) / 2 : ZH;
-    record_range<ZI, XP, SOFT, false>(p, rec, t % 32, lanes, z0, pairs, 0, 0, p.n_atoms, gx, gy, acc, [&]() {
+    record_range<ZI, XP, record_soft(PREC, SOFT), false>(p, rec, t % 32, lanes, z0, pairs, 0, 0, p.n_atoms, gx, gy, acc,
+                                                         [&]() {
         if constexpr (PREC != kPrecFp32) {
 #pragma unroll
             for (int k = 0; k < XP; ++k)
@@ -830,8 +840,9 @@ __global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel
     const int64_t w = static_cast<int64_t>(rank) * GROUP + gw;
     const int64_t a0 = (partials / shares * w + partials % shares * w / shares) * kRecordMerge;
     const int64_t stop = (partials / shares * (w + 1) + partials % shares * (w + 1) / shares) * kRecordMerge;
-    record_range<ZI, XP, SOFT, true>(p, rec, lane, 32, z0, (planes + 1) / 2, plane0 % ZI / depth, a0,
-                                     stop < p.n_atoms ? stop : p.n_atoms, gx, gy, acc, [&]() {
+    record_range<ZI, XP, record_soft(kPrecFp64Merge, SOFT), true>(p, rec, lane, 32, z0, (planes + 1) / 2,
+                                                                  plane0 % ZI / depth, a0,
+                                                                  stop < p.n_atoms ? stop : p.n_atoms, gx, gy, acc, [&]() {
 #pragma unroll
         for (int m = 0; m < ZI; ++m) {
             if (m < planes) {

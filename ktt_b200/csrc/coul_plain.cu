@@ -21,7 +21,7 @@
 // Bound: the MUFU unit and the FMA pipe together (5/16 of the reciprocal square roots on the FMA
 // pipe in 3D, 2/8 in 2D).  On B200, against the default configuration's tile (128 x 4 x 16 points in
 // 3D, 128 x 16 in 2D, all roots on MUFU): 37 x 41 x 33 x 211 atoms 15 us a call against 87; 96^3 x
-// 4,096 0.63 ms against 1.39; 256^3 x 16,384 6.1 Tpair/s against 4.4; a 250 x 187 slice x 1,501 30
+// 4,096 0.644 ms against 1.39; 200^3 x 8,000 5.9 Tpair/s against 3.2; a 250 x 187 slice x 1,501 32
 // against 176 us (with the conversion of its atoms).  What a thread's 32 points give in 3D: 16 points
 // (8 planes) reach 5.4.  100 registers and 16 warps an SM: 80 registers (24 warps)
 // spill a little and are 1 % slower, two atoms at a time are no faster.
@@ -39,10 +39,12 @@ namespace {
 
 constexpr int kPlainWarps = 8;
 constexpr int kPlainThreads = 32 * kPlainWarps;
-// Below this many atoms every reciprocal square root stays on MUFU: the FMA-pipe root's error (2.3e-7
-// rms) would show where the sums are too short to round more than that (211 atoms: 0.9e-7 of the
-// map's norm; the default configuration's single sum 2.9e-7), and such maps are bound by latency.
-constexpr int kPlainSoftAtoms = 512;
+// The share of a call without a configuration, of 16 roots in 3D and of 8 in 2D, at MUFU's precision (rsqrt_full):
+// 96^3 x 4,096 takes 644 us with 5/16 (2/16 745, 3/16 705, 4/16 659, 6/16 664; with
+// rsqrt_fma, good to 4.6e-7 only, 629), 96^3 x 400 76 us (no share 94), a 1024 x 1024 slice x 20,000 3.83 ms with 2/8
+// (1/8 or 3/8 4.19; rsqrt_fma 3.68).
+constexpr int kPlainSoft = 5;
+constexpr int kPlain2dSoft = 2;
 constexpr int kPlainMaxSplit = 8;  // portable cluster size
 
 // 3D: 2 x 16 points a thread; soft pairs spread over a thread's 16 lane pairs, SOFT of 16.
@@ -117,7 +119,7 @@ __device__ __forceinline__ void reduce_tile(float (*s)[P * 32], const int rows, 
 }
 
 // 3D: `cnt` staged atoms against the tile's first D planes.
-template <int SOFT, int D>
+template <int SOFT, int D>  // SOFT: sixteenths (+ kSoftFull)
 __device__ __forceinline__ void plain_batch(const float4* rec, const int cnt, const float (&gx)[kPlainX], const float gy,
                                             float2 (&acc)[kPlainX][kPlainZ / 2])
 {
@@ -142,10 +144,10 @@ __device__ __forceinline__ void plain_batch(const float4* rec, const int cnt, co
 #pragma unroll
             for (int m = 0; m < D / 2; ++m) {
                 const float2 r2 = __ffma2_rn(dz[m], dz[m], dxy);
-                if (SOFT != 0 && spread_soft(k * ZH + m, SOFT))
-                    acc[k][m] = __ffma2_rn(qs, rsqrt_fma_x2(r2), acc[k][m]);
+                if (SOFT != 0 && spread_soft(k * ZH + m, soft_share(SOFT)))
+                    pair_update<true, SOFT >= kSoftFull, false>(r2, q, qs, acc[k][m]);
                 else
-                    acc[k][m] = __ffma2_rn(q, rsqrt_mufu_x2(r2), acc[k][m]);
+                    pair_update<false, false, false>(r2, q, qs, acc[k][m]);
             }
         }
     }
@@ -365,6 +367,7 @@ int launch_plain_3d(coul_ctx* ctx, const FwdParams& f, int nz, int soft)
     case 6: kernel = plain_3d_kernel<6>; break;
     case 8: kernel = plain_3d_kernel<8>; break;
     case 10: kernel = plain_3d_kernel<10>; break;
+    case kPlainSoft + kSoftFull: kernel = plain_3d_kernel<kPlainSoft + kSoftFull>; break;
     default: return set_error(COUL_ERR_UNSUPPORTED, "no kernel for this share of FMA-pipe roots");
     }
     PlainParams p{};
@@ -418,7 +421,7 @@ COUL_API int coul_forward_3d_plain(coul_ctx* ctx, const float* d_atoms, int64_t 
     f.oz = grid->origin[2];
     f.out = d_out;
     f.accumulate = accumulate ? 1 : 0;
-    if ((rc = ctx_begin_timing(ctx)) || (rc = launch_plain_3d(ctx, f, grid->nz, n_atoms < kPlainSoftAtoms ? 0 : 5)))
+    if ((rc = ctx_begin_timing(ctx)) || (rc = launch_plain_3d(ctx, f, grid->nz, kPlainSoft + kSoftFull)))
         return rc;
     return ctx_end_timing(ctx);
 }
@@ -448,7 +451,7 @@ COUL_API int coul_forward_2d_plain(coul_ctx* ctx, const float* d_atoms, int64_t 
     const int64_t tiles = (static_cast<int64_t>(p.columns) * ((ny + kPlain2dY - 1) / kPlain2dY) + 31) / 32;
     const int split = plain_split(ctx, tiles, n_atoms, 4);
     if ((rc = ctx_begin_timing(ctx)) ||
-        (rc = launch_plain(ctx, n_atoms < kPlainSoftAtoms ? plain_2d_kernel<0> : plain_2d_kernel<2>, p, tiles, 1, split)))
+        (rc = launch_plain(ctx, plain_2d_kernel<kPlain2dSoft + kSoftFull>, p, tiles, 1, split)))
         return rc;
     return ctx_end_timing(ctx);
 }

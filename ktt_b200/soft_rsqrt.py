@@ -27,6 +27,10 @@ emulates the FP32 operation sequence exactly (products of two FP32 values are ex
 fused multiply-add is formed in FP64 and rounded once to FP32, which differs from a true FP32 fma
 only on FP64 double-rounding ties).
 
+``rsqrt_full`` is the device's second root, at MUFU's precision: y = magic(x), e = x y^2 - 1, result
+y + y e (c1 + c2 e + c3 e^2 + c4 e^3), the minimax polynomial of (1 + e)^(-1/2) - 1 without constant term on
+the constant's interval |e| < 0.0686 (Lawson's reweighted least squares, ``fit_full``).  2 integer + 7 FP32.
+
     python -m ktt_b200.soft_rsqrt            # exhaustive bound of the shipped constants
     python -m ktt_b200.soft_rsqrt --search   # re-derive the constants (about a minute)
 """
@@ -40,6 +44,9 @@ MAGIC = 0x5F1ED000
 A1 = np.float32(2.3597500324)
 A2 = np.float32(5.8324427605)
 SCALE = np.float32(0.1844490021)
+
+FULL_MAGIC = 0x5F375000
+FULL_C = tuple(np.float32(c) for c in (-0.49999833, 0.3749989, -0.31393645, 0.27455508))
 
 LOMONT = 0x5F375A86
 
@@ -65,6 +72,46 @@ def rsqrt_fma(x, magic: int = MAGIC, a1=A1, a2=A2) -> np.ndarray:
     x = np.asarray(x, dtype=np.float32)
     x64 = x.astype(np.float64)
     return _step(_step(_magic(x, magic), x64, a1), x64, a2)
+
+
+def _fma(a: np.ndarray, b, c) -> np.ndarray:
+    return (a.astype(np.float64) * np.asarray(b, dtype=np.float64) + np.asarray(c, dtype=np.float64)).astype(np.float32)
+
+
+def rsqrt_full(x) -> np.ndarray:
+    """FP32 emulation of the device's full-precision root."""
+    x = np.asarray(x, dtype=np.float32)
+    y = _magic(x, FULL_MAGIC)
+    e = _fma(x, (y * y).astype(np.float32), -1.0)
+    c = _fma(e, FULL_C[3], FULL_C[2])
+    c = _fma(c, e, FULL_C[1])
+    c = _fma(c, e, FULL_C[0])
+    return _fma(y, (e * c).astype(np.float32), y)
+
+
+def full_error_profile(step: int = 1) -> tuple[float, float]:
+    """(min, max) relative error of rsqrt_full(x) against 1/sqrt(x) over x in [1, 4)."""
+    x = _binade_pair(step)
+    e = rsqrt_full(x).astype(np.float64) * np.sqrt(x.astype(np.float64)) - 1.0
+    return float(e.min()), float(e.max())
+
+
+def fit_full() -> np.ndarray:
+    """c1..c4 for FULL_MAGIC."""
+    x = _binade_pair(97)
+    s = _magic(x, FULL_MAGIC).astype(np.float64) ** 2 * x
+    lo, hi = s.min() - 1.0, s.max() - 1.0
+    e = 0.5 * (lo + hi) + 0.5 * (hi - lo) * np.cos(np.linspace(0.0, np.pi, 4001))
+    a = np.stack([e ** k for k in range(1, 5)], 1) * np.sqrt(1.0 + e)[:, None]
+    b = 1.0 - np.sqrt(1.0 + e)
+    w = np.ones_like(e)
+    for _ in range(1000):
+        root = np.sqrt(w)
+        c = np.linalg.lstsq(a * root[:, None], b * root, rcond=None)[0]
+        r = np.abs(a @ c - b)
+        w *= r / r.max() + 1e-12
+        w /= w.sum()
+    return c
 
 
 def rsqrt_textbook(x) -> np.ndarray:

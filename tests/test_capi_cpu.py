@@ -121,3 +121,17 @@ def test_fma_pipe_rsqrt_bound_and_constants_match_device_code():
     for name, val in (("A1", sr.A1), ("A2", sr.A2), ("Scale", sr.SCALE)):
         m = re.search(rf"kSoftRsqrt{name} = ([0-9.eE+-]+)f;", src)
         assert m and np.float32(float(m.group(1))) == val, name
+
+
+def test_full_fma_pipe_rsqrt_bound_and_constants_match_device_code():
+    """The FMA-pipe root at MUFU's precision: exhaustive FP32 bound over every input in [1, 4) below
+    rsqrt.approx's documented 2^-22.9, and the device header's constants."""
+    from ktt_b200 import soft_rsqrt as sr
+    lo, hi = sr.full_error_profile()
+    assert -2.0**-22.9 < lo < 0 < hi < 2.0**-22.9
+    assert np.max(np.abs(sr.fit_full() - np.array(sr.FULL_C, dtype=np.float64))) < 1e-6
+    src = open(os.path.join(REPO, "ktt_b200", "csrc", "coul_device.cuh")).read()
+    assert f"kFullRsqrtMagic = {sr.FULL_MAGIC:#x}u" in src
+    for i, val in enumerate(sr.FULL_C):
+        m = re.search(rf"kFullRsqrtC{i + 1} = ([0-9.eE+-]+)f;", src)
+        assert m and np.float32(float(m.group(1))) == val, i

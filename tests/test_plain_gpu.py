@@ -197,3 +197,35 @@ def test_atoms_closer_than_the_range_of_the_root(ctx, n):
             a[7] = ((0.0, 0.0, r, 1.0), (r, 0.0, 0.0, 1.0))[k % 2]
             got = ctx.forward_3d(_cuda(a), (96, 64, 32), 0.5, origin)[k // 2, 0, k % 2].item()
             assert got == want or abs(got / want - 1) <= 1e-6, (k, r)
+
+
+@pytest.mark.parametrize("fields", [None, dict(z_iterations=16, x_points=2, rsqrt_soft=12, precision=2),
+                                    dict(z_iterations=16, x_points=2, rsqrt_soft=2, precision=4)])
+def test_root_of_one_pair_at_mufu_precision(ctx, fields):
+    """One charge of 1 among 600 charge-free atoms, every coordinate a multiple of 1/16 below 64: differences of
+    10 bits, r^2 exact in FP32, the sum the root itself.  rsqrt.approx's documented bound, 2^-22.9, holds for every
+    root of a call whose caller did not choose another; with FP64 sums also in a batch."""
+    rng = np.random.default_rng(5)
+    dims, h = (80, 64, 48), 0.5
+    gz, gy, gx = np.meshgrid(*(np.arange(d) * h for d in dims[::-1]), indexing="ij")
+    tune = ktt_b200.Tune(block_x=16, block_y=2, **fields) if fields else None
+    for i in range(8):
+        a = np.zeros((600, 4), dtype=np.float32)
+        a[:, :3] = (2 * rng.integers(0, 8 * 32, (600, 3)) + 1) / 16
+        j = int(rng.integers(0, 600))
+        a[j, 3] = 1.0
+        exact = 1.0 / np.sqrt((gx - a[j, 0]) ** 2 + (gy - a[j, 1]) ** 2 + (gz - a[j, 2]) ** 2)
+        maps = [ctx.forward_3d(_cuda(a), dims, h, tune=tune).cpu().numpy()]
+        if fields and fields["precision"] == 4:
+            batch = ktt_b200.Batch(ctx, [(_cuda(a), dims, h, (0.0, 0.0, 0.0))],
+                                   ktt_b200.Tune(block_x=8, block_y=4, **dict(fields, rsqrt_soft=12)))
+            batch.run()
+            ctx.synchronize()
+            maps.append(batch.outputs[0].cpu().numpy())
+            batch.close()
+        if fields is None:
+            flat = a.copy()
+            flat[:, 2] = a[:, 2] ** 2
+            maps.append(ctx.forward_2d(_cuda(flat), h, dims[0], dims[1]).cpu().numpy())
+        for v in maps:
+            assert np.max(np.abs(v / (exact if v.ndim == 3 else exact[0]) - 1)) <= 2.0**-22.9 + 2.0**-30
