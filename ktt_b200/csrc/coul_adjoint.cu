@@ -8,8 +8,8 @@
 // transposed sum.  A thread owns one atom, a CTA kAdjThreads atoms and a chunk of grid rows; the rows'
 // G values pass through shared memory in blocks of kRows rows x X points, and while a block of
 // X columns is processed the thread holds its X differences dx = x - a.x in registers, so a
-// pair costs six FP32 operations -- r^2 = fma(dx, dx, dy^2 + dz^2), 1/r^2, 1/r^3, and three FMAs that
-// add G/r (for the charge), G/r^3 by column (its sum times dx gives the x component) and G/r^3 by row
+// pair costs six FP32 operations -- r^2 = fma(dx, dx, dy^2 + dz^2), t = G/r, 1/r^2, the sum of t (for the
+// charge), and two FMAs that add t/r^2 by column (its sum times dx gives the x component) and by row
 // (its sum times dy and dz gives the other two) -- and one MUFU rsqrt.  Two neighbouring columns share
 // each packed instruction: dx, the column sums and the four-point loads of G come in pairs as they
 // are.  The FP32 sums of one block go into FP64 sums per atom; each (atom tile, row chunk) writes its
@@ -148,10 +148,11 @@ __global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoin
                     const float2 g = m & 1 ? make_float2(gq.z, gq.w) : make_float2(gq.x, gq.y);
                     const float2 r2 = __ffma2_rn(dx[m], dx[m], dyz2);
                     const float2 inv = rsqrt_mufu_x2(r2);
-                    const float2 inv3 = __fmul2_rn(__fmul2_rn(inv, inv), inv);
-                    sq[m % kChains] = __ffma2_rn(g, inv, sq[m % kChains]);
-                    s3x[m] = __ffma2_rn(g, inv3, s3x[m]);
-                    s3r = m == 0 ? __fmul2_rn(g, inv3) : __ffma2_rn(g, inv3, s3r);
+                    const float2 t = __fmul2_rn(g, inv);  // not 1/r^3 first: it leaves FP32's range before G/r^3 does
+                    const float2 inv2 = __fmul2_rn(inv, inv);
+                    sq[m % kChains] = __fadd2_rn(sq[m % kChains], t);
+                    s3x[m] = __ffma2_rn(t, inv2, s3x[m]);
+                    s3r = m == 0 ? __fmul2_rn(t, inv2) : __ffma2_rn(t, inv2, s3r);
                 }
                 const float v = s3r.x + s3r.y;
                 sy = fmaf(dy, v, sy);

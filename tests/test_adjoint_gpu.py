@@ -211,3 +211,39 @@ def test_adjoint_block_edges(ctx, dims, n):
     got = got.cpu().numpy().astype(np.float64)
     assert _rel(got[:, 3], dq) <= 1e-5
     assert _rel(got[:, :3], dr) <= 1e-5
+
+
+def _gradient_fp64(atoms, dims, h, grad_map):
+    """dL/dq and dL/dr of every atom with G = grad_map, in FP64; a point with G = 0 adds nothing."""
+    g = [np.arange(d, dtype=np.float64) * h for d in dims]
+    points = np.stack([c.ravel() for c in np.meshgrid(*g[::-1], indexing="ij")], 1)[:, ::-1]
+    w = grad_map.astype(np.float64).ravel()
+    points, w = points[w != 0], w[w != 0]
+    dq, dr = np.empty(atoms.shape[0]), np.empty((atoms.shape[0], 3))
+    for j, a in enumerate(atoms.astype(np.float64)):
+        d = points - a[:3]
+        r = np.sqrt((d * d).sum(1))
+        dq[j] = (w / r).sum()
+        dr[j] = a[3] * ((w / r ** 3)[:, None] * d).sum(0)
+    return dq, dr
+
+
+@pytest.mark.parametrize("dims", [(8, 4, 4), (40, 6, 5), (64, 3, 3)])
+def test_adjoint_masked_point_close_to_an_atom(ctx, dims):
+    """A point with G = 0 (a fit's mask) adds nothing however close the atom lies: 1 / r^3 leaves FP32's range
+    below 1.4e-13, G / r * (1 / r^2) does not before r^2 does.  An FP32 pair chain is good to about 4e-7: 1e-5."""
+    import torch
+    rng = np.random.default_rng(dims[0])
+    atoms = np.empty((40, 4), dtype=np.float32)
+    atoms[:, :3] = rng.uniform(-3.0, 3.0, (40, 3))
+    atoms[:, 3] = rng.uniform(0.2, 1.0, 40)
+    for j, r in enumerate((1e-13, 1e-14, 1e-16, 2e-18)):
+        atoms[j, :3] = np.roll((r, 0.0, 0.0), j % 3)  # next to the origin's point
+    grad_map = rng.uniform(0.5, 1.0, dims[::-1]).astype(np.float32)
+    grad_map[0, 0, 0] = 0.0
+    dq, dr = _gradient_fp64(atoms, dims, 0.5, grad_map)
+    got = ktt_b200.adjoint_3d(ctx, torch.from_numpy(atoms).cuda(), dims, 0.5, torch.from_numpy(grad_map).cuda())
+    got = got.cpu().numpy().astype(np.float64)
+    assert np.all(np.isfinite(got))
+    assert _rel(got[:, 3], dq) <= 1e-5
+    assert _rel(got[:, :3], dr) <= 1e-5
