@@ -12,13 +12,19 @@
 // charge), and two FMAs that add t/r^2 by column (its sum times dx gives the x component) and by row
 // (its sum times dy and dz gives the other two) -- and one MUFU rsqrt.  Two neighbouring columns share
 // each packed instruction: dx, the column sums and the four-point loads of G come in pairs as they
-// are.  The FP32 sums of one block go into FP64 sums per atom; each (atom tile, row chunk) writes its
-// FP64 partials, and a second kernel adds the chunks in a fixed order, so the result is deterministic.
+// are.  A row is summed by itself, the rows of a block are added in FP32 and the block's sums go into FP64
+// sums per atom; each (atom tile, row chunk) writes its FP64 partials, and a second kernel adds the
+// chunks in a fixed order, so the result is deterministic.
+//
+// An FP32 sum is thus no longer than a row of 25 points and more: chains of a row's 16 lane pairs (8), then of
+// the block's 8 rows (16); column sums of 16 rows.  Rows of up to 24 points (SHORT) would not be: theirs go
+// into FP64 one by one, and G dx/r^3 is added along the row (eight operations a pair).  With rows of 64 terms
+// in one chain the charge gradient was 1.2 to 1.7 times less exact than row by row for nx <= 32.
 //
 // Bound: the MUFU unit (one rsqrt a pair at 16 a clock and SM, 4.64e12 pairs/s; the six FP32
-// operations alone would allow 5.9e12).  128^3 x 8,192 atoms: 4.2 ms = 4.07 Tpair/s, the MUFU
-// unit 89 % busy, against 4.85 ms for a form with the atoms in pairs, eight FP32 operations a pair and
-// whole rows per thread; 61 x 57 x 50 x 777 atoms: 56 us for the call against 174.
+// operations alone would allow 5.9e12).  128^3 x 8,192 atoms: 4.38 ms = 3.93 Tpair/s, against 4.86 ms for a form
+// with the atoms in pairs, eight FP32 operations a pair and whole rows per thread; 61 x 57 x 50 x 777 atoms: 59 us
+// for the call against 174; rows of 1 point, 447 x 447 of them, x 3,000 atoms: 1.30 ms against 1.75.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,19 +36,17 @@ namespace coul {
 
 constexpr int kAdjThreads = 128;
 
-// Shapes of the kernel by the grid columns X a thread holds in registers: rows per staged block,
-// chains of the block's FP32 charge sum (64 and 32 terms a lane: with 128 the charge gradient is less
-// exact than one row of 64 at a time) and resident CTAs per SM.  32 columns share a row's dy^2 + dz^2,
-// its sums and its loads of G among twice as many pairs: 4.07 Tpair/s on 128^3 x 8,192 against 3.93
-// with 16, which stay for row lengths that 32 would pad (16 warps of 124 registers against 20 of 92;
-// 8 columns: 3.64, two atoms a thread with 8 columns: 3.63).
-template <int X>
+// Shapes of the kernel by the grid columns X a thread holds in registers: rows per staged block and resident
+// CTAs per SM.  32 columns share a row's dy^2 + dz^2, its sums and its loads of G among twice as many pairs as
+// 16, which stay for row lengths that 32 would pad (16 warps of 126 registers against 20 of 94).  SHORT, us with
+// 3,000 atoms and 200,000 points, against the form with whole rows per thread: 4 columns, rows of 1, 2, 4 points
+// 1,300, 660, 340 (1,744, 1,044, 668); 8, rows of 8 256 (502); 16, rows of 16 211 (418); 24, rows of 24 205 (393).
+template <int X, bool SHORT>
 struct AdjShape {
-    static constexpr int kRows = 256 / X;
-    static constexpr int kChains = X == 32 ? 2 : 4;
-    static constexpr int kBlocksPerSm = X == 32 ? 4 : 5;
+    static constexpr int kRows = X == 24 ? 16 : 256 / X;
+    static constexpr int kBlocksPerSm = X == 32 ? 4 : SHORT && X < 24 ? 6 : 5;
 };
-constexpr int kAdjFoldRows = 64;   // terms of a column sum before it goes into FP64
+constexpr int kAdjFoldRows = 16;  // terms of a column sum before it goes into FP64
 constexpr int kAdjReduceWarps = 8;
 
 struct AdjParams {
@@ -56,12 +60,12 @@ struct AdjParams {
     int chunks;
 };
 
-template <int X>
-__global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoint_kernel(const AdjParams p)
+template <int X, bool SHORT>
+__global__ void __launch_bounds__(kAdjThreads, AdjShape<X, SHORT>::kBlocksPerSm) adjoint_kernel(const AdjParams p)
 {
-    constexpr int kRows = AdjShape<X>::kRows;
-    constexpr int kChains = AdjShape<X>::kChains;
+    constexpr int kRows = AdjShape<X, SHORT>::kRows;
     constexpr int M = X / 2;                              // lane pairs of columns
+    constexpr int C = SHORT ? 2 : 1;                      // chains of a row's sums
     constexpr int kPerThread = kRows * X / kAdjThreads;   // staged values per thread
     static_assert(kRows * X % kAdjThreads == 0 && X % 4 == 0 && kRows <= kAdjThreads, "block shape");
     // two buffers: a block is staged while slower warps still read the one before, one barrier a block
@@ -105,13 +109,14 @@ __global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoin
         }
         // the column sums into FP64: at the end of the rows, and every kAdjFoldRows rows
         auto fold_x = [&]() {
-            float2 sx = make_float2(0.0f, 0.0f);
+            float2 sx[4];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                sx = __ffma2_rn(dx[m], s3x[m], sx);
+                sx[m % 4] = m < 4 ? __fmul2_rn(dx[m], s3x[m]) : __ffma2_rn(dx[m], s3x[m], sx[m % 4]);
                 s3x[m] = make_float2(0.0f, 0.0f);
             }
-            tx += static_cast<double>(sx.x + sx.y);
+            const float2 sum = __fadd2_rn(__fadd2_rn(sx[0], sx[1]), __fadd2_rn(sx[2 % M], sx[3 % M]));
+            tx += static_cast<double>(sum.x + sum.y);
         };
         int unfolded = 0;
         for (int64_t row0 = r_begin; row0 < r_end; row0 += kRows) {
@@ -130,10 +135,7 @@ __global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoin
                 fetch(row0 + kRows, x0);
             else
                 fetch(r_begin, x0 + X);
-            float2 sq[kChains];
-#pragma unroll
-            for (int i = 0; i < kChains; ++i)
-                sq[i] = make_float2(0.0f, 0.0f);
+            float2 sq = make_float2(0.0f, 0.0f);
             float sy = 0.0f, sz = 0.0f;
             for (int r = 0; r < count; ++r) {
                 const float2 yz = s_row[buf][r];
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoin
                 const float dz = yz.y - a.z;
                 const float2 dyz2 = splat(fmaf(dy, dy, dz * dz));
                 const float4* g4 = reinterpret_cast<const float4*>(s_g[buf] + r * X);
-                float2 s3r = make_float2(0.0f, 0.0f);
+                float2 q[C], s3[C], sx[C];  // the row's sums
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     const float4 gq = g4[m / 2];
@@ -150,28 +152,44 @@ __global__ void __launch_bounds__(kAdjThreads, AdjShape<X>::kBlocksPerSm) adjoin
                     const float2 inv = rsqrt_mufu_x2(r2);
                     const float2 t = __fmul2_rn(g, inv);  // not 1/r^3 first: it leaves FP32's range before G/r^3 does
                     const float2 inv2 = __fmul2_rn(inv, inv);
-                    sq[m % kChains] = __fadd2_rn(sq[m % kChains], t);
-                    s3x[m] = __ffma2_rn(t, inv2, s3x[m]);
-                    s3r = m == 0 ? __fmul2_rn(t, inv2) : __ffma2_rn(t, inv2, s3r);
+                    q[m % C] = m < C ? t : __fadd2_rn(q[m % C], t);
+                    if constexpr (SHORT) {
+                        const float2 t3 = __fmul2_rn(t, inv2);
+                        s3[m % C] = m < C ? t3 : __fadd2_rn(s3[m % C], t3);
+                        sx[m % C] = m < C ? __fmul2_rn(t3, dx[m]) : __ffma2_rn(t3, dx[m], sx[m % C]);
+                    } else {
+                        s3x[m] = __ffma2_rn(t, inv2, s3x[m]);
+                        s3[m % C] = m < C ? __fmul2_rn(t, inv2) : __ffma2_rn(t, inv2, s3[m % C]);
+                    }
                 }
-                const float v = s3r.x + s3r.y;
-                sy = fmaf(dy, v, sy);
-                sz = fmaf(dz, v, sz);
+                const float2 qr = SHORT ? __fadd2_rn(q[0], q[C - 1]) : q[0];
+                const float2 v2 = SHORT ? __fadd2_rn(s3[0], s3[C - 1]) : s3[0];
+                const float v = v2.x + v2.y;
+                if constexpr (SHORT) {
+                    const float2 xr = __fadd2_rn(sx[0], sx[C - 1]);
+                    tq += static_cast<double>(qr.x + qr.y);
+                    tx += static_cast<double>(xr.x + xr.y);
+                    ty = fma(static_cast<double>(dy), static_cast<double>(v), ty);
+                    tz = fma(static_cast<double>(dz), static_cast<double>(v), tz);
+                } else {
+                    sq = __fadd2_rn(sq, qr);
+                    sy = fmaf(dy, v, sy);
+                    sz = fmaf(dz, v, sz);
+                }
             }
-            float2 q = sq[0];
-#pragma unroll
-            for (int i = 1; i < kChains; ++i)
-                q = __fadd2_rn(q, sq[i]);
-            tq += static_cast<double>(q.x + q.y);
-            ty += static_cast<double>(sy);
-            tz += static_cast<double>(sz);
-            unfolded += kRows;
-            if (unfolded == kAdjFoldRows) {
-                fold_x();
-                unfolded = 0;
+            if constexpr (!SHORT) {
+                tq += static_cast<double>(sq.x + sq.y);
+                ty += static_cast<double>(sy);
+                tz += static_cast<double>(sz);
+                unfolded += kRows;
+                if (unfolded >= kAdjFoldRows) {
+                    fold_x();
+                    unfolded = 0;
+                }
             }
         }
-        fold_x();
+        if constexpr (!SHORT)
+            fold_x();
     }
     if (j < p.n_atoms) {
         double2* dst = reinterpret_cast<double2*>(p.partial + (static_cast<int64_t>(blockIdx.y) * p.n_atoms + j) * 4);
@@ -226,10 +244,31 @@ struct AdjointWorkspace {
 
 using namespace coul;
 
-template <int X>
+template <int X, bool SHORT>
 static void launch_adjoint(const AdjParams& p, int64_t tiles, cudaStream_t stream)
 {
-    adjoint_kernel<X><<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(p.chunks)), kAdjThreads, 0, stream>>>(p);
+    adjoint_kernel<X, SHORT><<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(p.chunks)), kAdjThreads, 0, stream>>>(p);
+}
+
+// The kernel for rows of nx points.
+struct AdjForm {
+    void (*launch)(const AdjParams&, int64_t, cudaStream_t);
+    int blocks_per_sm;
+};
+
+template <int X, bool SHORT>
+static AdjForm adjoint_form()
+{
+    return AdjForm{&launch_adjoint<X, SHORT>, AdjShape<X, SHORT>::kBlocksPerSm};
+}
+
+static AdjForm adjoint_form(int64_t nx)
+{
+    if (nx <= 24)  // the fewest columns that hold a row
+        return nx <= 4 ? adjoint_form<4, true>() : nx <= 8 ? adjoint_form<8, true>() : nx <= 16 ? adjoint_form<16, true>() : adjoint_form<24, true>();
+    // 32 columns a thread unless they pad the rows by more than the 4 % they gain over 16
+    const auto padded = [&](int64_t x) { return (nx + x - 1) / x * x; };
+    return padded(32) * 100 <= padded(16) * 104 ? adjoint_form<32, false>() : adjoint_form<16, false>();
 }
 
 // The call of both entry points: any of the three outputs may be NULL.
@@ -251,13 +290,11 @@ static int adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, cons
 
     const int64_t tiles = (n_atoms + kAdjThreads - 1) / kAdjThreads;
     const int64_t rows = static_cast<int64_t>(grid->ny) * grid->nz;
-    // 32 columns a thread unless they pad the rows by more than the 4 % they gain over 16
-    const auto padded = [&](int64_t x) { return (grid->nx + x - 1) / x * x; };
-    const bool wide = padded(32) * 100 <= padded(16) * 104;
+    const AdjForm form = adjoint_form(grid->nx);
     // Equal (tile, chunk) CTAs in whole waves of the resident ones, rounded down so that no wave is
     // nearly empty: as many waves (at most 8; the SMs' warps drift apart within one) as leave a chunk
     // 32 rows, else one wave.
-    const int64_t slots = static_cast<int64_t>(ctx->sm_count) * (wide ? AdjShape<32>::kBlocksPerSm : AdjShape<16>::kBlocksPerSm);
+    const int64_t slots = static_cast<int64_t>(ctx->sm_count) * form.blocks_per_sm;
     int64_t chunks = 1;
     for (int64_t waves = 8; waves >= 1; --waves) {
         chunks = std::max<int64_t>(1, waves * slots / tiles);
@@ -312,10 +349,7 @@ static int adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, cons
     p.chunks = static_cast<int>(chunks);
     if ((rc = ctx_begin_timing(ctx)))
         return rc;
-    if (wide)
-        launch_adjoint<32>(p, tiles, ctx->stream);
-    else
-        launch_adjoint<16>(p, tiles, ctx->stream);
+    form.launch(p, tiles, ctx->stream);
     if ((e = cudaGetLastError()) != cudaSuccess)
         return cuda_error(e, "adjoint launch");
     adjoint_reduce_kernel<<<static_cast<unsigned>((n_atoms + 7) / 8), 32 * kAdjReduceWarps, 0, ctx->stream>>>(

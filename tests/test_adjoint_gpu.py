@@ -247,3 +247,44 @@ def test_adjoint_masked_point_close_to_an_atom(ctx, dims):
     assert np.all(np.isfinite(got))
     assert _rel(got[:, 3], dq) <= 1e-5
     assert _rel(got[:, :3], dr) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 128, 300])
+@pytest.mark.parametrize("dims", [(1, 90, 7), (2, 65, 1), (3, 9, 8), (4, 64, 65), (5, 33, 2), (8, 32, 9), (9, 17, 3),
+                                  (16, 16, 17), (17, 5, 16), (23, 7, 7), (24, 33, 16), (25, 8, 9), (47, 17, 1)])
+def test_adjoint_short_rows(ctx, dims, n):
+    """Rows around the kernel's widths (4, 8, 16, 24, then blocks of 16 and 32), row counts around its staged blocks
+    (64, 32, 16, 8), against the FP64 gradient.  G in [0.5, 1]: the charge sums do not cancel, the position sums by
+    less than a factor of ten in the largest component: 1e-5 as above."""
+    import torch
+    rng = np.random.default_rng(1000 * n + dims[0])
+    atoms = np.empty((n, 4), dtype=np.float32)
+    atoms[:, :3] = rng.uniform(-4.0, 0.5 * max(dims) + 4.0, (n, 3))
+    atoms[:, 3] = rng.uniform(0.2, 1.0, n)
+    grad_map = rng.uniform(0.5, 1.0, dims[::-1]).astype(np.float32)
+    dq, dr = _gradient_fp64(atoms, dims, 0.5, grad_map)
+    got = ktt_b200.adjoint_3d(ctx, torch.from_numpy(atoms).cuda(), dims, 0.5, torch.from_numpy(grad_map).cuda())
+    got = got.cpu().numpy().astype(np.float64)
+    assert _rel(got[:, 3], dq) <= 1e-5
+    assert _rel(got[:, :3], dr) <= 1e-5
+
+
+@pytest.mark.parametrize("nx", [1, 2, 3, 4])
+def test_adjoint_short_rows_are_summed_in_fp64(ctx, nx):
+    """Charge gradient of rows of a few points, G normal.  Rounding errors in units of u = 2^-24, rms of a rounding
+    0.42 u (uniform over a binade): differences and r^2 0.42 and 0.36, the root 1 (documented below 2.15), G / r and the
+    store 0.42 each, together 1.3 u; a row's sum adds 0.42 u times the square root of its log2(nx) levels, and FP64
+    sums of rows add nothing.  Sums of 64 rows in FP32 would come to 1.6 u and more."""
+    import torch
+    u = 2.0**-24
+    rng = np.random.default_rng(nx)
+    ny = int((200_000 // nx) ** 0.5)
+    dims = (nx, ny, ny)
+    atoms = np.empty((200, 4), dtype=np.float32)
+    atoms[:, :3] = rng.uniform(0.0, 1.0, (200, 3)) * 0.5 * np.array(dims)
+    atoms[:, 3] = rng.uniform(-1.0, 1.0, 200)
+    grad_map = rng.normal(0.0, 1.0, dims[::-1]).astype(np.float32)
+    dq, _ = _gradient_fp64(atoms, dims, 0.5, grad_map)
+    got = ktt_b200.adjoint_3d(ctx, torch.from_numpy(atoms).cuda(), dims, 0.5, torch.from_numpy(grad_map).cuda())
+    error = np.linalg.norm(got[:, 3].cpu().numpy().astype(np.float64) - dq) / np.linalg.norm(dq)
+    assert error <= u * np.sqrt(1.3**2 + 0.42**2 * np.log2(nx))
