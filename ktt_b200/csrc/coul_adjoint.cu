@@ -235,11 +235,6 @@ __global__ void __launch_bounds__(32 * kAdjReduceWarps) adjoint_reduce_kernel(
         grad_xyz[3 * j + k - 1] = v;
 }
 
-struct AdjointWorkspace {
-    double* partial = nullptr;
-    size_t bytes = 0;
-};
-
 }  // namespace coul
 
 using namespace coul;
@@ -307,31 +302,12 @@ static int adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, cons
     if (tiles > 2147483647LL)
         return set_error(COUL_ERR_DEVICE_LIMITS, "too many atoms");
 
-    // Workspace for the FP64 partials, kept in the context and grown on demand.
-    static_assert(sizeof(AdjointWorkspace) > 0, "");
-    auto* ws = static_cast<AdjointWorkspace*>(ctx->adjoint_workspace);
-    if (ws == nullptr) {
-        ws = new AdjointWorkspace();
-        ctx->adjoint_workspace = ws;
-        ctx->cleanups.push_back([ws] {
-            if (ws->partial)
-                cudaFree(ws->partial);
-            delete ws;
-        });
-    }
-    const size_t need = static_cast<size_t>(chunks) * static_cast<size_t>(n_atoms) * 4 * sizeof(double);
-    cudaError_t e;
-    if (need > ws->bytes) {
-        if (ws->partial) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(ws->partial);
-            ws->partial = nullptr;
-            ws->bytes = 0;
-        }
-        if ((e = cudaMalloc(&ws->partial, need)) != cudaSuccess)
-            return set_error(COUL_ERR_OUT_OF_MEMORY, std::string("adjoint workspace: ") + cudaGetErrorString(e));
-        ws->bytes = need;
-    }
+    void* partial = nullptr;
+    bool own = false;
+    if ((rc = workspace_begin(ctx, kWorkspaceAdjoint,
+                              static_cast<size_t>(chunks) * static_cast<size_t>(n_atoms) * 4 * sizeof(double), "adjoint",
+                              &partial, &own)))
+        return rc;
 
     AdjParams p{};
     p.atoms = reinterpret_cast<const float4*>(d_atoms);
@@ -344,18 +320,19 @@ static int adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, cons
     p.oy = grid->origin[1];
     p.oz = grid->origin[2];
     p.grad_map = d_grad_map;
-    p.partial = ws->partial;
+    p.partial = static_cast<double*>(partial);
     p.rows_per_chunk = rows_per_chunk;
     p.chunks = static_cast<int>(chunks);
     if ((rc = ctx_begin_timing(ctx)))
-        return rc;
+        return workspace_fail(ctx, rc);
+    cudaError_t e;
     form.launch(p, tiles, ctx->stream);
     if ((e = cudaGetLastError()) != cudaSuccess)
-        return cuda_error(e, "adjoint launch");
+        return workspace_fail(ctx, cuda_error(e, "adjoint launch"));
     adjoint_reduce_kernel<<<static_cast<unsigned>((n_atoms + 7) / 8), 32 * kAdjReduceWarps, 0, ctx->stream>>>(
-        p.atoms, ws->partial, n_atoms, p.chunks, d_grad_q, d_grad_xyz, reinterpret_cast<float4*>(d_grad));
+        p.atoms, p.partial, n_atoms, p.chunks, d_grad_q, d_grad_xyz, reinterpret_cast<float4*>(d_grad));
     if ((e = cudaGetLastError()) != cudaSuccess)
-        return cuda_error(e, "adjoint reduction launch");
+        return workspace_fail(ctx, cuda_error(e, "adjoint reduction launch"));
     return ctx_end_timing(ctx);
 }
 

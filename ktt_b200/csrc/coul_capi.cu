@@ -225,11 +225,19 @@ int ctx_begin_timing(coul_ctx* ctx)
 
 int ctx_end_timing(coul_ctx* ctx)
 {
-    if (ctx->timing_held)
+    Workspace* const ws = ctx->open_workspace;
+    if (ctx->timing_held && ws == nullptr)
         return COUL_OK;
-    cudaError_t e = cudaEventRecord(ctx->ev_stop, ctx->stream);
+    ctx->open_workspace = nullptr;
+    const cudaEvent_t stop = ws ? ws->used : ctx->ev_stop;
+    cudaError_t e = cudaEventRecord(stop, ctx->stream);
     if (e != cudaSuccess)
         return cuda_error(e, "cudaEventRecord");
+    if (ws)
+        ws->recorded = true;
+    if (ctx->timing_held)
+        return COUL_OK;
+    ctx->last_stop = stop;
     ctx->have_timing = true;
     return COUL_OK;
 }
@@ -712,6 +720,7 @@ COUL_API int coul_ctx_destroy(coul_ctx* ctx)
     if (ctx->stream)
         cudaStreamSynchronize(ctx->stream);
     orphan_batches(ctx);
+    release_workspaces(ctx);
     if (ctx->d_atoms_cache)
         cudaFree(ctx->d_atoms_cache);
     if (ctx->d_out_cache)
@@ -838,11 +847,11 @@ COUL_API int coul_elapsed_ms(coul_ctx* ctx, double* ms)
         return set_error(COUL_ERR_INVALID_ARGUMENT, "ctx or ms is NULL");
     if (!ctx->have_timing)
         return set_error(COUL_ERR_INVALID_ARGUMENT, "no timed call yet");
-    cudaError_t e = cudaEventSynchronize(ctx->ev_stop);
+    cudaError_t e = cudaEventSynchronize(ctx->last_stop);
     if (e != cudaSuccess)
         return cuda_error(e, "cudaEventSynchronize");
     float f = 0.0f;
-    e = cudaEventElapsedTime(&f, ctx->ev_start, ctx->ev_stop);
+    e = cudaEventElapsedTime(&f, ctx->ev_start, ctx->last_stop);
     if (e != cudaSuccess)
         return cuda_error(e, "cudaEventElapsedTime");
     *ms = static_cast<double>(f);

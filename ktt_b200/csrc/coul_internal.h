@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,27 @@ struct coul_batch;
 
 constexpr int kHostSlabs = 16;  // slabs of a host-buffer call (at most)
 
+namespace coul {
+
+struct CaptureBuffer;
+
+// A buffer of coul_workspace.cu's.
+struct Workspace {
+    void* mem = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t used = nullptr;  // the end of its last use
+    bool recorded = false;       // `used` has been recorded since the memory was had
+    // The balanced form's counters (at the start of the memory, one per CTA) are known to be zero for
+    // this many CTAs (0: unknown).  Its kernel leaves them at zero when it completes, so a following
+    // launch of the same grid needs no reset; the queue form's use of the memory, a reallocation or
+    // a kernel that failed or timed out clears this.
+    int64_t clean = 0;
+};
+
+enum WorkspaceKind { kWorkspaceAdjoint, kWorkspaceSplit, kWorkspacePairs, kWorkspaceKinds };
+
+}  // namespace coul
+
 struct coul_ctx {
     int device = 0;
     void* user_context = nullptr;  // the caller's CUcontext (coul_ctx_create_on), else the primary context
@@ -21,6 +43,7 @@ struct coul_ctx {
     cudaStream_t stream = nullptr;  // the stream every call of this context is enqueued on
     cudaEvent_t ev_start = nullptr; // bracket the most recent timed call
     cudaEvent_t ev_stop = nullptr;
+    cudaEvent_t last_stop = nullptr;  // the last call's end: ev_stop or its workspace's event
     bool have_timing = false;
     bool timing_held = false;       // a call of several launches records the events itself
     // host-buffer calls in slabs (created by the first): every other slab's stream, the copies' stream, the
@@ -37,7 +60,9 @@ struct coul_ctx {
     int cc_major = 0;
     int cc_minor = 0;
     std::vector<std::function<void()>> cleanups;  // frees buffers owned by other units (run at destroy)
-    void* adjoint_workspace = nullptr;            // FP64 partials of coul_adjoint_3d (coul_adjoint.cu)
+    coul::Workspace workspaces[coul::kWorkspaceKinds];  // coul_workspace.cu
+    coul::Workspace* open_workspace = nullptr;          // that of the call in progress
+    std::vector<std::shared_ptr<coul::CaptureBuffer>> capture_buffers;  // of captured calls
     void* split_workspace_state = nullptr;        // partial blocks and counters of the queue and balanced forms
     void* nbody_workspace = nullptr;              // partial accelerations of the pair form (coul_nbody.cu)
     std::vector<coul_batch*> batches;             // live batches (their device resources go with the context)
@@ -57,6 +82,12 @@ int cuda_error(cudaError_t e, const char* what);
 int ctx_activate(coul_ctx* ctx);
 int ctx_begin_timing(coul_ctx* ctx);
 int ctx_end_timing(coul_ctx* ctx);
+// `need` bytes for the call in progress, ordered after their last use (coul_workspace.cu).  *own: the call is
+// captured and the memory is its graph's alone (nothing is known of its contents).  ctx_end_timing ends the use; a
+// call that fails after this returns through workspace_fail.
+int workspace_begin(coul_ctx* ctx, WorkspaceKind kind, size_t need, const char* what, void** mem, bool* own);
+int workspace_fail(coul_ctx* ctx, int rc);
+void release_workspaces(coul_ctx* ctx);
 bool aligned16(const void* p);
 int validate_tune(const coul_tune* t, int mode, int soa, const VariantEntry** out);
 int validate_grid(const coul_grid* g);

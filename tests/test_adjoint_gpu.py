@@ -288,3 +288,57 @@ def test_adjoint_short_rows_are_summed_in_fp64(ctx, nx):
     got = ktt_b200.adjoint_3d(ctx, torch.from_numpy(atoms).cuda(), dims, 0.5, torch.from_numpy(grad_map).cuda())
     error = np.linalg.norm(got[:, 3].cpu().numpy().astype(np.float64) - dq) / np.linalg.norm(dq)
     assert error <= u * np.sqrt(1.3**2 + 0.42**2 * np.log2(nx))
+
+
+def test_adjoint_on_two_streams_and_captured(ctx):
+    """The context's partial sums are one stream's at a time (gradients of two sizes on two streams, nothing waited
+    for between); captured calls, on two streams forked within one capture as well, keep memory of their own: their
+    replays equal the eager calls bit for bit after later calls have grown the context's, beside eager calls on another
+    stream, and for a second graph made when the first is gone."""
+    import torch
+    rng = np.random.default_rng(12)
+    data, want = [], []
+    for n, dims in ((3000, (61, 57, 50)), (700, (40, 90, 33))):
+        atoms = np.empty((n, 4), dtype=np.float32)
+        atoms[:, :3] = rng.uniform(0.0, 25.0, (n, 3))
+        atoms[:, 3] = rng.uniform(-1.0, 1.0, n)
+        g = rng.normal(0.0, 1.0, dims[::-1]).astype(np.float32)
+        data.append((torch.from_numpy(atoms).cuda(), dims, 0.5, torch.from_numpy(g).cuda()))
+        want.append(ktt_b200.adjoint_3d(ctx, *data[-1]))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def eager():
+        got = []
+        for i in range(8):
+            with torch.cuda.stream(streams[i % 2]):
+                got.append((i % 2, ktt_b200.adjoint_3d(ctx, *data[i % 2])))
+        return got
+
+    got = eager()
+    torch.cuda.synchronize()
+    for k, grad in got:
+        assert torch.equal(grad, want[k])
+    for _ in range(2):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            fork, side = torch.cuda.current_stream(), torch.cuda.Stream()
+            first = ktt_b200.adjoint_3d(ctx, *data[0])
+            side.wait_stream(fork)
+            with torch.cuda.stream(side):
+                beside = [ktt_b200.adjoint_3d(ctx, *data[1]) for _ in range(2)]
+            again = ktt_b200.adjoint_3d(ctx, *data[0])
+            fork.wait_stream(side)
+        big = torch.cat([data[0][0]] * 8)
+        ktt_b200.adjoint_3d(ctx, big, *data[0][1:])
+        for _ in range(3):
+            for out in (first, again, *beside):
+                out.zero_()
+            graph.replay()
+            got = eager()
+            torch.cuda.synchronize()
+            assert torch.equal(first, want[0]) and torch.equal(again, want[0])
+            assert all(torch.equal(b, want[1]) for b in beside)
+            for k, grad in got:
+                assert torch.equal(grad, want[k])
+        del graph, first, again, beside
