@@ -301,18 +301,6 @@ int validate_grid(const coul_grid* g)
     return COUL_OK;
 }
 
-// Device memory of the queue and balanced forms of the atom split, kept in the context and grown on
-// demand: partial blocks and counters (the layout is each form's own).
-struct SplitWorkspace {
-    void* mem = nullptr;
-    size_t bytes = 0;
-    // The balanced form's counters (at the start of the memory, one per CTA) are known to be zero for
-    // this many CTAs (0: unknown).  Its kernel leaves them at zero when it completes, so a following
-    // launch of the same grid needs no reset; the queue form's use of the memory, a reallocation or
-    // a timed-out kernel clears this.
-    int64_t balanced_clean_ctas = 0;
-};
-
 // Resident blocks per SM of a persistent form's kernel for this block size and dynamic shared memory.
 // The kernel's dynamic shared-memory attribute is only ever raised (never lowered, by any context
 // object sharing the CUDA context), so every size launched before stays launchable.  Queried once per
@@ -340,36 +328,6 @@ static int resident_blocks(coul_ctx* ctx, const void* kernel, int threads, size_
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kernel, threads, smem)) != cudaSuccess)
         return cuda_error(e, "occupancy query");
     ctx->occupancy_cache.push_back(coul_ctx::Occupancy{kernel, threads, smem, *blocks});
-    return COUL_OK;
-}
-
-// Grow the context's split workspace to `need` bytes (drains the stream before freeing the old one).
-static int split_workspace(coul_ctx* ctx, size_t need, unsigned char** base)
-{
-    auto* ws = static_cast<SplitWorkspace*>(ctx->split_workspace_state);
-    if (ws == nullptr) {
-        ws = new SplitWorkspace();
-        ctx->split_workspace_state = ws;
-        ctx->cleanups.push_back([ws] {
-            if (ws->mem)
-                cudaFree(ws->mem);
-            delete ws;
-        });
-    }
-    if (need > ws->bytes) {
-        ws->balanced_clean_ctas = 0;
-        if (ws->mem) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(ws->mem);
-            ws->mem = nullptr;
-            ws->bytes = 0;
-        }
-        cudaError_t e;
-        if ((e = cudaMalloc(&ws->mem, need)) != cudaSuccess)
-            return set_error(COUL_ERR_OUT_OF_MEMORY, std::string("atom-split workspace: ") + cudaGetErrorString(e));
-        ws->bytes = need;
-    }
-    *base = static_cast<unsigned char*>(ws->mem);
     return COUL_OK;
 }
 
@@ -405,15 +363,18 @@ int balanced_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, con
     const size_t done_bytes = static_cast<size_t>(ctas) * sizeof(unsigned);
     const size_t partial_offset = (done_bytes + 255) / 256 * 256;
     const size_t need = partial_offset + static_cast<size_t>(2 * ctas * values) * sizeof(float);
-    unsigned char* base = nullptr;
-    const int rc = split_workspace(ctx, need, &base);
-    if (rc != COUL_OK)
+    void* mem = nullptr;
+    bool own = false;
+    if (const int rc = workspace_begin(ctx, kWorkspaceSplit, need, "atom-split", &mem, &own))
         return rc;
-    auto* ws = static_cast<SplitWorkspace*>(ctx->split_workspace_state);
-    if (ws->balanced_clean_ctas != ctas) {
+    auto* base = static_cast<unsigned char*>(mem);
+    // a captured call resets its counters on every replay, which may follow one that gave up
+    Workspace& ws = ctx->workspaces[kWorkspaceSplit];
+    if (own || ws.clean != ctas) {
         if ((e = cudaMemsetAsync(base, 0, done_bytes, ctx->stream)) != cudaSuccess)
-            return cuda_error(e, "balanced form counters reset");
-        ws->balanced_clean_ctas = ctas;
+            return workspace_fail(ctx, cuda_error(e, "balanced form counters reset"));
+        if (!own)
+            ws.clean = ctas;
     }
     L.queue.partial = reinterpret_cast<float*>(base + partial_offset);
     L.queue.tile_done = reinterpret_cast<unsigned*>(base);
@@ -433,20 +394,22 @@ int queue_split_setup(coul_ctx* ctx, const VariantEntry* v, FwdLaunch& L, const 
     const size_t done_offset = (partial_bytes + 255) / 256 * 256;
     const size_t counter_offset = (done_offset + static_cast<size_t>(tiles) * sizeof(unsigned) + 255) / 256 * 256;
     const size_t need = counter_offset + 256;
-    unsigned char* base = nullptr;
-    const int rc = split_workspace(ctx, need, &base);
-    if (rc != COUL_OK)
-        return rc;
-    static_cast<SplitWorkspace*>(ctx->split_workspace_state)->balanced_clean_ctas = 0;
-    cudaError_t e;
-    // the per-tile counters and the queue head start every launch at zero
-    if ((e = cudaMemsetAsync(base + done_offset, 0, need - done_offset, ctx->stream)) != cudaSuccess)
-        return cuda_error(e, "queue counters reset");
     int blocks_per_sm = 0;
     if (const int rc_occ = resident_blocks(ctx, v->occupancy_kernel, threads, L.smem, &blocks_per_sm))
         return rc_occ;
     if (blocks_per_sm < 1)
         return set_error(COUL_ERR_DEVICE_LIMITS, "the queue form's block does not fit on an SM");
+    void* mem = nullptr;
+    bool own = false;
+    if (const int rc = workspace_begin(ctx, kWorkspaceSplit, need, "atom-split", &mem, &own))
+        return rc;
+    auto* base = static_cast<unsigned char*>(mem);
+    if (!own)
+        ctx->workspaces[kWorkspaceSplit].clean = 0;
+    cudaError_t e;
+    // the per-tile counters and the queue head start every launch at zero
+    if ((e = cudaMemsetAsync(base + done_offset, 0, need - done_offset, ctx->stream)) != cudaSuccess)
+        return workspace_fail(ctx, cuda_error(e, "queue counters reset"));
     L.queue.partial = reinterpret_cast<float*>(base);
     L.queue.tile_done = reinterpret_cast<unsigned*>(base + done_offset);
     L.queue.counter = reinterpret_cast<unsigned long long*>(base + counter_offset);
@@ -603,9 +566,9 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
                       : 0;
     cudaError_t e = v->launch(L, ctx->stream);
     if (e == cudaErrorLaunchOutOfResources)
-        return set_error(COUL_ERR_DEVICE_LIMITS, std::string("forward launch: ") + cudaGetErrorString(e));
+        return workspace_fail(ctx, set_error(COUL_ERR_DEVICE_LIMITS, std::string("forward launch: ") + cudaGetErrorString(e)));
     if (e != cudaSuccess)
-        return cuda_error(e, "forward launch");
+        return workspace_fail(ctx, cuda_error(e, "forward launch"));
     return COUL_OK;
 }
 
@@ -833,8 +796,7 @@ COUL_API int coul_synchronize(coul_ctx* ctx)
         return cuda_error(e, "status read-back");
     if (status != kStatusOk) {
         cudaMemset(ctx->d_status, 0, sizeof(int));
-        if (ctx->split_workspace_state)  // a kernel that gave up may have left counters behind
-            static_cast<SplitWorkspace*>(ctx->split_workspace_state)->balanced_clean_ctas = 0;
+        ctx->workspaces[kWorkspaceSplit].clean = 0;  // a kernel that gave up may have left counters behind
         return set_error(COUL_ERR_TIMEOUT, "a kernel gave up on a bounded wait (status " + std::to_string(status) +
                                                "); its output is invalid");
     }

@@ -246,3 +246,50 @@ def test_balanced_split_alternating_sizes_and_contexts(ctx):
             first.setdefault(key, got)
     finally:
         other.close()
+
+
+@pytest.mark.parametrize("form", [1, 2])
+def test_split_workspace_on_two_streams_and_captured(ctx, form):
+    """The queue and balanced forms' partial blocks and counters are one stream's at a time (slices of two sizes on two
+    streams, nothing waited for between); a captured call has its own: captured before any eager call, its replays
+    equal the eager calls bit for bit, also after a larger call has grown the context's memory and beside eager
+    calls on another stream, and the eager calls after a capture find their counters at zero."""
+    import torch
+    rng = np.random.default_rng(form)
+    own = ktt_b200.CoulombContext(0)
+    sizes = ((100, 90, 3000), (64, 200, 1100))
+    tunes = [ktt_b200.Tune(block_x=32, block_y=1, z_iterations=4, x_points=4, unroll=2, rsqrt_soft=2, atom_split=s,
+                           split_form=form) for s in ((32, 16) if form == 2 else (12, 7))]
+    atoms = [torch.from_numpy(rng.uniform(0.1, 30.0, (n, 4)).astype(np.float32)).cuda() for _, _, n in sizes]
+    want = [ctx.forward_2d(atoms[k], 0.5, sizes[k][0], sizes[k][1], tune=tunes[k]) for k in range(2)]
+    torch.cuda.synchronize()
+
+    def call(k):
+        return own.forward_2d(atoms[k], 0.5, sizes[k][0], sizes[k][1], tune=tunes[k])
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        first, again, other = call(0), call(0), call(1)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def eager():
+        got = []
+        for i in range(8):
+            with torch.cuda.stream(streams[i % 2]):
+                got.append((i % 2, call(i % 2)))
+        return got
+
+    for attempt in range(3):
+        if attempt == 1:
+            own.forward_2d(atoms[0], 0.25, 700, 500, tune=tunes[0])
+            torch.cuda.synchronize()
+        for out in (first, again, other):
+            out.zero_()
+        graph.replay()
+        got = eager()
+        torch.cuda.synchronize()
+        assert torch.equal(first, want[0]) and torch.equal(again, want[0]) and torch.equal(other, want[1])
+        for k, out in got:
+            assert torch.equal(out, want[k])
+    del graph
+    own.close()
