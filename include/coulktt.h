@@ -346,8 +346,11 @@ COUL_API int coul_nbody_tune_supported(const coul_nbody_tune* tune);
 COUL_API int coul_nbody_step(coul_ctx* ctx, const float* d_pos_mass, const float* d_vel, int64_t n, float dt,
                              float damping, float softening_sqr, const coul_nbody_tune* tune, float* d_pos_mass_new,
                              float* d_vel_new);
-/* The same step without a configuration: a kernel that suits every body count (csrc/coul_nbody.cu).  No
-   counterpart in the reference, whose tuner picks a configuration for every launch. */
+/* The same step without a configuration: kernels that suit every body count (csrc/coul_nbody.cu).  From 4,096
+   bodies on each pair is evaluated once for both, with a workspace of at most 256 MB that the context keeps; beyond
+   about 183,000 bodies, where it would be larger, where it is not to be had and under stream capture, each side by
+   itself without one (0.72 of the rate).  No counterpart in the reference, whose tuner picks a configuration for every
+   launch. */
 COUL_API int coul_nbody_step_plain(coul_ctx* ctx, const float* d_pos_mass, const float* d_vel, int64_t n, float dt,
                                    float damping, float softening_sqr, float* d_pos_mass_new, float* d_vel_new);
 

@@ -63,7 +63,6 @@ struct coul_ctx {
     coul::Workspace workspaces[coul::kWorkspaceKinds];  // coul_workspace.cu
     coul::Workspace* open_workspace = nullptr;          // that of the call in progress
     std::vector<std::shared_ptr<coul::CaptureBuffer>> capture_buffers;  // of captured calls
-    void* nbody_workspace = nullptr;              // partial accelerations of the pair form (coul_nbody.cu)
     std::vector<coul_batch*> batches;             // live batches (their device resources go with the context)
     struct Occupancy {
         const void* kernel;

@@ -719,21 +719,13 @@ COUL_API int coul_nbody_step(coul_ctx* ctx, const float* d_pos_mass, const float
     return ctx_end_timing(ctx);
 }
 
-// The pair form's workspace, kept in the context and grown on demand.
-struct PairWorkspace {
-    float* mem = nullptr;
-    size_t bytes = 0;
-    cudaEvent_t used = nullptr;     // recorded after each use ...
-    cudaStream_t stream = nullptr;  // ... on this stream; another stream waits for it
-};
-
 // From this many bodies on the pair form is faster than the one-way kernel (10,000
 // bodies: 60 us, 65; 131,072: 5.17 ms, 7.16).
 constexpr int64_t kPairBodies = 4096;
 constexpr size_t kPairWorkspaceLimit = size_t{256} << 20;
 
 // The pair form of the plain step.  Sets *done when it was launched; otherwise the caller launches the
-// one-way kernel, which needs no workspace: under stream capture (a graph would keep the pointer), beyond
+// one-way kernel, which needs no workspace: under stream capture (a graph would hold as much again), beyond
 // the workspace limit, or when the memory is not to be had.
 static int nbody_pairs(coul_ctx* ctx, const NbodyParams& n, bool* done)
 {
@@ -757,51 +749,22 @@ static int nbody_pairs(coul_ctx* ctx, const NbodyParams& n, bool* done)
         cudaGetLastError();
         return COUL_OK;
     }
-    auto* ws = static_cast<PairWorkspace*>(ctx->nbody_workspace);
-    if (ws == nullptr) {
-        ws = new PairWorkspace();
-        ctx->nbody_workspace = ws;
-        ctx->cleanups.push_back([ws] {
-            if (ws->mem)
-                cudaFree(ws->mem);
-            if (ws->used)
-                cudaEventDestroy(ws->used);
-            delete ws;
-        });
-    }
+    void* mem = nullptr;
+    bool own = false;
+    int rc = workspace_begin(ctx, kWorkspacePairs, need, "N-body", &mem, &own);
+    if (rc != COUL_OK)
+        return rc == COUL_ERR_OUT_OF_MEMORY ? COUL_OK : rc;
+    p.own = static_cast<float*>(mem);
+    p.by_distance = p.own + static_cast<size_t>(p.parts) * 3 * static_cast<size_t>(p.padded);
+    if ((rc = ctx_begin_timing(ctx)))
+        return workspace_fail(ctx, rc);
     cudaError_t e;
-    if (ws->used == nullptr && (e = cudaEventCreateWithFlags(&ws->used, cudaEventDisableTiming)) != cudaSuccess)
-        return cuda_error(e, "N-body workspace event");
-    if (need > ws->bytes) {
-        if (ws->mem) {
-            cudaEventSynchronize(ws->used);
-            cudaFree(ws->mem);
-            ws->mem = nullptr;
-            ws->bytes = 0;
-        }
-        if (cudaMalloc(&ws->mem, need) != cudaSuccess) {
-            cudaGetLastError();
-            ws->mem = nullptr;
-            return COUL_OK;
-        }
-        ws->bytes = need;
-        ws->stream = ctx->stream;
-    } else if (ws->stream != ctx->stream) {
-        if ((e = cudaStreamWaitEvent(ctx->stream, ws->used, 0)) != cudaSuccess)
-            return cuda_error(e, "N-body workspace order");
-        ws->stream = ctx->stream;
-    }
-    p.own = ws->mem;
-    p.by_distance = ws->mem + static_cast<size_t>(p.parts) * 3 * static_cast<size_t>(p.padded);
-    int rc = ctx_begin_timing(ctx);
-    if (rc)
-        return rc;
     nbody_pair_kernel<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(p.parts)), 32 * kStepWarps, 0, ctx->stream>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess)
-        return cuda_error(e, "N-body launch");
+        return workspace_fail(ctx, cuda_error(e, "N-body launch"));
     nbody_gather_kernel<<<static_cast<unsigned>(p.padded / 32), 256, 0, ctx->stream>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaEventRecord(ws->used, ctx->stream)) != cudaSuccess)
-        return cuda_error(e, "N-body launch");
+    if ((e = cudaGetLastError()) != cudaSuccess)
+        return workspace_fail(ctx, cuda_error(e, "N-body launch"));
     *done = true;
     return ctx_end_timing(ctx);
 }

@@ -132,3 +132,51 @@ def test_nbody_plain_step_on_two_streams_and_captured(ctx):
     torch.cuda.synchronize()
     # two summation orders of an acceleration, times dt: 1e-5 of the largest velocity covers both
     assert float((out[1] - want[1][1]).abs().max()) <= 1e-5 * float(want[1][1].abs().max())
+
+
+@pytest.mark.parametrize("n", [180_000, 186_000])
+def test_nbody_plain_step_around_the_workspace_limit(ctx, n):
+    """The pair form up to the workspace's 256 MB (about 183,000 bodies) and the one-way kernel beyond, 64 seeded
+    bodies checked."""
+    import torch
+    pos, vel = _bodies(n, seed=n)
+    p, v = ktt_b200.nbody_step(ctx, torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda(), DT, DAMPING, EPS2)
+    idx = np.sort(np.random.default_rng(3).choice(n, 64, replace=False))
+    _check(pos, vel, p.cpu().numpy(), v.cpu().numpy(), idx)
+
+
+def test_nbody_plain_step_beside_a_capture(ctx):
+    """A context's first pair-form step, which allocates, while another thread captures a stream in the strictest mode:
+    the capture goes on, and the step is the pair form's bit for bit."""
+    import threading
+
+    import torch
+    pos, vel = _bodies(9000, seed=2)
+    tp, tv = torch.from_numpy(pos).cuda(), torch.from_numpy(vel).cuda()
+    want = ktt_b200.nbody_step(ctx, tp, tv, DT, DAMPING, EPS2)
+    out = [torch.empty_like(tp), torch.empty_like(tv)]
+    fresh = ktt_b200.CoulombContext(0)
+    stream = torch.cuda.Stream()
+    x = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    failed = []
+
+    def step():
+        try:
+            with torch.cuda.stream(stream):
+                ktt_b200.nbody_step(fresh, tp, tv, DT, DAMPING, EPS2, out_pos=out[0], out_vel=out[1])
+        except Exception as e:  # noqa: BLE001 (reported by the test)
+            failed.append(e)
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x += 1.0
+        worker = threading.Thread(target=step)
+        worker.start()
+        worker.join()
+        x += 1.0
+    assert not failed
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1]) and float(x[0]) == 2.0
+    fresh.close()
