@@ -495,6 +495,19 @@ static bool plain_tile(const coul_ctx* ctx, const VariantEntry* v, const coul_tu
     return tiles_xy * ((nz + 15) / 16) < 64LL * ctx->sm_count;
 }
 
+// Blocks of a configuration's launch over nx x ny x nz points, or a refusal where a grid cannot hold them.
+static int launch_blocks(const coul_tune* t, int mode, int nx, int ny, int nz, int64_t* gx, int64_t* gy, int64_t* gz)
+{
+    const auto blocks = [](int64_t points, int64_t per_block) { return (points + per_block - 1) / per_block; };
+    const bool map = mode == kModeGrid3d;
+    *gx = blocks(nx, static_cast<int64_t>(t->block_x) * t->x_points);
+    *gy = blocks(ny, static_cast<int64_t>(t->block_y) * (map ? 1 : t->z_iterations));
+    *gz = map ? blocks(nz, t->z_iterations) : 1;
+    if (*gx > 2147483647LL || *gy > 65535 || *gz > 65535)
+        return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
+    return COUL_OK;
+}
+
 // Launch one forward variant over a grid; shared by the 3D AoS/SoA and 2D entry points and by
 // the batched path's plain-launch baseline.
 int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, int mode, const coul_tune* t, int nz)
@@ -503,19 +516,9 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
     L.p = prm;
     L.p.status = ctx->d_status;
     L.block = dim3(static_cast<unsigned>(t->block_x), static_cast<unsigned>(t->block_y), 1);
-    const int64_t bx = static_cast<int64_t>(t->block_x) * t->x_points;
-    const int64_t gx = (prm.nx + bx - 1) / bx;
-    int64_t gy, gz;
-    if (mode == kModeGrid3d) {
-        gy = (prm.ny + t->block_y - 1) / t->block_y;
-        gz = (prm.nz - prm.z_base + t->z_iterations - 1) / t->z_iterations;
-    } else {
-        const int64_t by = static_cast<int64_t>(t->block_y) * t->z_iterations;
-        gy = (prm.ny + by - 1) / by;
-        gz = 1;
-    }
-    if (gx > 2147483647LL || gy > 65535 || gz > 65535)
-        return set_error(COUL_ERR_DEVICE_LIMITS, "grid too large for one launch");
+    int64_t gx, gy, gz;
+    if (const int rc = launch_blocks(t, mode, prm.nx, prm.ny, prm.nz - prm.z_base, &gx, &gy, &gz))
+        return rc;
     if (plain_tile(ctx, v, t, mode, prm, nz)) {
         const int soft = t->rsqrt_soft;
         return launch_plain_3d(ctx, prm, nz, soft >= kSoftAlternate ? 2 * (soft - kSoftAlternate) + 1 : 2 * soft);
@@ -1206,7 +1209,12 @@ static int forward_3d_host(coul_ctx* ctx, const float* h_atoms, int64_t n_atoms,
     if (abytes > 0 &&
         (e = cudaMemcpyAsync(ctx->d_atoms_cache, h_atoms, abytes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_error(e, "atom upload");
-    if (const int planes = slab_planes(grid, n_atoms, tune); planes < grid->nz)
+    const int planes = slab_planes(grid, n_atoms, tune);
+    int64_t gx, gy, gz;
+    if (tune && planes < grid->nz &&  // a map too deep for the configuration is so in slabs too
+        (rc = launch_blocks(tune, kModeGrid3d, grid->nx, grid->ny, grid->nz, &gx, &gy, &gz)))
+        return rc;
+    if (planes < grid->nz)
         return host_slabs(ctx, n_atoms, grid, tune, planes, h_out);
     rc = tune ? coul_forward_3d(ctx, ctx->d_atoms_cache, n_atoms, grid, tune, 0, ctx->d_out_cache)
               : coul_forward_3d_plain(ctx, ctx->d_atoms_cache, n_atoms, grid, 0, grid->nz, 0, ctx->d_out_cache);

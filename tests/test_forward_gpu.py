@@ -448,3 +448,17 @@ def test_fp64_pairs_on_a_column_deeper_than_one_grid(ctx):
     out = _np(ctx.forward_3d(_t(a), dims, 1.0, tune=tune))
     ref = oracle.grid3d(a, 1.0, dims)
     assert np.max(np.abs(out - ref) / np.abs(ref)) <= 1.2e-7
+
+
+def test_host_buffer_call_refuses_what_the_device_call_refuses(ctx):
+    """A map of more planes of tiles than a grid holds is refused as a whole, also where the host-buffer call would
+    have cut it into slabs that fit."""
+    a = np.zeros((2000, 4), dtype=np.float32)
+    tune = ktt_b200.Tune(block_x=32, block_y=1, z_iterations=1, x_points=1)
+    dims = (16, 1, 70_000)
+    with pytest.raises(ktt_b200.CoulombError) as e:
+        ctx.forward_3d(_t(a), dims, 0.5, tune=tune)
+    assert e.value.status == ktt_b200.COUL_ERR_DEVICE_LIMITS
+    with pytest.raises(ktt_b200.CoulombError) as e:
+        ctx.forward_3d_host(a, dims, 0.5, tune=tune)
+    assert e.value.status == ktt_b200.COUL_ERR_DEVICE_LIMITS
