@@ -429,22 +429,23 @@ static void record_split_setup(const coul_ctx* ctx, FwdLaunch& L, const coul_tun
     const int64_t tiles_xy = (static_cast<int64_t>(columns) * L.p.ny + 31) / 32;
     const auto tiles_at = [&](int depth) { return tiles_xy * ((nz + depth - 1) / depth); };
     const int64_t tiles = tiles_at(zi);
-    const int64_t partials = (L.p.n_atoms + kRecordMerge - 1) / kRecordMerge;
-    // Warps per tile: more until the map has 54 of them an SM (16 are resident: three to four rounds), and
-    // beyond that while each keeps 13 partials.  us by warps per tile (1, 2, 4, 8) on B200: 128^3 x 500 atoms
-    // 233, 230, 212, 221; 64^3 x 500 90, 74, 45, 42; 224^3 x 300 608, 625, 661, 688; 224^3 x 5,000 9,798,
-    // 9,741, 9,710, 9,626.
+    const int64_t n = L.p.n_atoms;
+    // Warps per tile: more until the map has 54 of them an SM (16 are resident: three to four rounds), and beyond
+    // that while each keeps some hundred atoms; none below 10 atoms a warp.  us by warps per tile (1, 2, 4, 8) on
+    // B200: 96^3 x 60 atoms 26, 26, 24, 28; 128^3 x 500 240, 230, 203, 205; 64^3 x 500 94, 74, 43, 40;
+    // 224^3 x 300 638, 634, 656, 670; x 700 1,455, 1,428, 1,441, 1,461; x 4,000 8,193, 7,949, 7,942, 7,858.
     int group = 1;
-    while (group < kRecordSplitWarps && (tiles * group < 54LL * ctx->sm_count || partials >= 26LL * group))
+    while (group < kRecordSplitWarps && n >= 20 * group &&
+           (tiles * group < 54LL * ctx->sm_count || n >= (group == 1 ? 400 : 750 * group)))
         group *= 2;
     if (group == 1)
         return;  // fwd_kernel
-    // half the depth, then more CTAs a tile, while there are fewer CTAs than SMs
+    // half the depth, then more CTAs a tile while there are fewer CTAs than SMs and a warp keeps 47 atoms
     const int per_cta = kRecordSplitWarps / group;
     const int depth = group == kRecordSplitWarps && tiles < ctx->sm_count ? zi / 2 : zi;
     int ranks = 1;
     while (group == kRecordSplitWarps && ranks < kMaxPortableSplit && tiles_at(depth) * ranks < ctx->sm_count &&
-           partials >= 2 * ranks * kRecordSplitWarps)
+           n >= 750LL * ranks)
         ranks *= 2;
     if (tiles_xy * ranks > 2147483647LL || (nz + depth - 1) / depth > 65535)
         return;

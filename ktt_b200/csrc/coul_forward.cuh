@@ -32,14 +32,14 @@ __device__ __forceinline__ double* shared_sums(unsigned char* tiles)
 }
 inline size_t shared_sums_bytes(int threads, int points) { return static_cast<size_t>(threads) * points * sizeof(double); }
 
-// Record tiles: with 2 x 16 points a thread, each warp of a 3D tile turns 24 atoms at a time into records
+// Record tiles: with 2 x 16 points a thread, each warp of a 3D tile turns 32 atoms at a time into records
 // in its own part of shared memory -- x, y, q, q * kSoftRsqrtScale and the atom's z differences to the
 // tile's 16 planes -- and evaluates them from there (record_accumulate), so the pair loop spends nothing
 // on dz and a thread's 32 points share what is left of an atom's cost.  Only tiles of this shape: with 16
 // points a thread the records' loads cost what they save (5.76 Tpair/s in a bare pair loop against
 // 5.87), with 64 the registers leave 12 warps an SM (5.88 against 6.30 with 32).
-constexpr int kRecordAtoms = 24;
-constexpr int kRecordMerge = 48;  // atoms per FP32 partial of the FP64-merge forms
+constexpr int kRecordAtoms = 32;
+constexpr int kRecordMerge = kMergeAtoms;  // atoms per FP32 partial of the FP64-merge forms, at most
 constexpr bool record_tile(const int zi, const int xp, const int src, const int soa, const int prec, const int mode)
 {
     return mode == kModeGrid3d && src == kSrcShared && soa == 0 && zi == 16 && xp == 2 &&
@@ -217,7 +217,7 @@ __device__ __forceinline__ void record_batch(const float4* rec, const int count,
     }
 }
 
-// The atoms [a0, a1) (a0 a multiple of kRecordMerge) through a warp's records in `rec`, the tile's planes
+// The atoms [a0, a1) through a warp's records in `rec`, the tile's planes
 // from z0 on, `pairs` pairs of them (of a whole tile, or with HALVES of its sub-th half); merge() after
 // every kRecordMerge atoms and at the end.  The lanes load the next batch of atoms into registers while
 // the warp evaluates the current one.
@@ -282,8 +282,8 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
 // The FMA-pipe roots of the FP64-merge record tiles are the full ones: five sixteenths of rsqrt_fma's, where 8 x 2
 // points had four, made the gradient of a fit 12 % (charges) and 5 % (positions) less exact (mean of 12 drawn fits).
 // Errors against 64 bits with 8 x 2 points and 4/16, 2 x 16 and 5/16 of rsqrt_fma, the same of rsqrt_full: 128^3 x
-// 8,192 2.58e-7, 2.49e-7, 1.77e-7; the fits' gradients 1, 1.12, 0.41 and 1, 1.05, 0.65; 12 to 32 molecules
-// 2.3e-7, 2.3e-7, 1.7e-7; 256^3 x 65,536 in 195.9, 186.4, 193.1 ms.
+// 8,192 2.58e-7, 2.49e-7, 2.05e-7; the fits' gradients 1, 1.12, 0.41 and 1, 1.05, 0.67; 32 molecules 2.34e-7, 2.28e-7,
+// 1.85e-7; 256^3 x 65,536 in 195.9, 186.3, 188.4 ms.
 constexpr int record_soft(const int prec, const int soft)
 {
     return prec == kPrecFp32 || soft == 0 ? soft : soft + kSoftFull;
@@ -291,8 +291,8 @@ constexpr int record_soft(const int prec, const int soft)
 
 // tile_accumulate for record tiles: a warp needs no other.  On 256^3 x 65,536 with 5/16 of the roots on
 // the FMA pipe: FP32 sums 180.1 ms = 6.10 Tpair/s (8 x 2 points through the TMA ring, 2/8: 191.8 ms), FP64
-// merge 193.1 ms = 5.69 Tpair/s (195.9; atoms split, record_split_kernel).  An FP32 partial of 48 atoms, not
-// kMergeAtoms: 72 and 96 are no faster (194.4, 193.4 ms) and less exact (128^3 x 8,192 1.77e-7, 2.03e-7, 2.44e-7).
+// merge 188.4 ms = 5.84 Tpair/s (195.9; atoms split, record_split_kernel).  FP32 partials of kMergeAtoms atoms in
+// batches of 32: partials of 48 in batches of 24 take 191.7 ms.
 template <int ZI, int XP, int PREC, int SOFT>
 __device__ __forceinline__ void record_accumulate(const FwdParams& p, const int x0, const int yrow, const int z0,
                                                   unsigned char* smem, float (&val)[XP][ZI])
@@ -787,14 +787,13 @@ __device__ __forceinline__ void store_split_sums(const FwdParams& p, double* all
 }
 
 // FP64-merge record tiles with their atoms split: GROUP (8, 4 or 2) of a CTA's eight warps, and with all
-// eight the CTAs of a cluster, share a tile of 32 linear columns by `depth` planes (ZI or half of it).
-// They split its atoms at multiples of kRecordMerge, so they form the FP32 partials of the whole tile and
-// only the FP64 additions of those take another order (warp order, then rank order): a point's float is
-// that of fwd_kernel unless its FP64 sum lies within a few units of the 53rd bit of a rounding boundary.
-// How a map is split follows from the whole grid and the atom count, so slabs equal the map bit for bit.
-// One warp a tile leaves a 128^3 map 3.5 warps a scheduler and its last ones alone (3,573 us x 8,192
-// atoms; split over eight 2,948), a 64^3 map half of the SMs idle (670 and 224 us x 4,000 atoms); even
-// 256^3 x 65,536 gains from the shorter tail (187.5 and 184.1 ms).
+// eight the CTAs of a cluster, share a tile of 32 linear columns by `depth` planes (ZI or half of it) and split its
+// atoms evenly, each share in FP32 partials of its own, their FP64 sums added in warp order, then in rank order.
+// How a map is split follows from the whole grid and the atom count, so slabs equal the map bit for bit; a point
+// differs from fwd_kernel's by the partials' rounding.  One warp a tile leaves a 128^3 map 3.5 warps a scheduler and
+// its last ones alone, a 64^3 map half of the SMs idle (700 and 236 us x 4,000 atoms); even 256^3 x 65,536 gains from
+// the shorter tail.  Shares of whole partials of 48 atoms left some warps a partial more than others: 128^3 x 250 131 us,
+// evenly 114 (8 x 2 points a thread 119), 61 x 190 x 100 x 100 68 and 43 (53), 128^3 x 8,192 3.10 and 3.02 ms.
 template <int ZI, int XP, int SOFT, int GROUP>
 __global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel(const FwdParams p, const int depth,
                                                                                 const int vec_ok)
@@ -834,15 +833,14 @@ __global__ void __launch_bounds__(32 * kRecordSplitWarps, 2) record_split_kernel
                 acc[k][i] = make_float2(0.0f, 0.0f);
     };
     clear();
-    // this warp's share: whole partials
-    const int64_t partials = (p.n_atoms + kRecordMerge - 1) / kRecordMerge;
+    // this warp's share
     const int64_t shares = static_cast<int64_t>(ranks) * GROUP;
     const int64_t w = static_cast<int64_t>(rank) * GROUP + gw;
-    const int64_t a0 = (partials / shares * w + partials % shares * w / shares) * kRecordMerge;
-    const int64_t stop = (partials / shares * (w + 1) + partials % shares * (w + 1) / shares) * kRecordMerge;
+    const int64_t a0 = p.n_atoms / shares * w + p.n_atoms % shares * w / shares;
+    const int64_t stop = p.n_atoms / shares * (w + 1) + p.n_atoms % shares * (w + 1) / shares;
     record_range<ZI, XP, record_soft(kPrecFp64Merge, SOFT), true>(p, rec, lane, 32, z0, (planes + 1) / 2,
                                                                   plane0 % ZI / depth, a0,
-                                                                  stop < p.n_atoms ? stop : p.n_atoms, gx, gy, acc, [&]() {
+                                                                  stop, gx, gy, acc, [&]() {
 #pragma unroll
         for (int m = 0; m < ZI; ++m) {
             if (m < planes) {

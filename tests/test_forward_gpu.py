@@ -462,3 +462,94 @@ def test_host_buffer_call_refuses_what_the_device_call_refuses(ctx):
     with pytest.raises(ktt_b200.CoulombError) as e:
         ctx.forward_3d_host(a, dims, 0.5, tune=tune)
     assert e.value.status == ktt_b200.COUL_ERR_DEVICE_LIMITS
+
+
+def _signed_atoms(n, seed, box):
+    rng = np.random.default_rng(seed)
+    a = np.empty((n, 4), dtype=np.float32)
+    a[:, :3] = rng.uniform(0.0, box, (n, 3))
+    a[:, 3] = rng.uniform(-1.0, 1.0, n)
+    return a
+
+
+@pytest.mark.parametrize("dims,n", [((96, 96, 96), 15), ((96, 96, 96), 30), ((96, 96, 96), 60), ((128, 128, 128), 73),
+                                    ((128, 128, 128), 250), ((131, 117, 125), 500), ((160, 160, 160), 97),
+                                    ((160, 160, 161), 250), ((224, 224, 224), 19), ((224, 224, 209), 60)])
+@pytest.mark.parametrize("prec", [ktt_b200.PREC_FP64_MERGE, ktt_b200.PREC_FP64_MERGE_SHARED])
+def test_record_tiles_by_warps_a_tile(ctx, dims, n, prec):
+    """FP64-merge record tiles with 1, 2, 4 and 8 warps a tile (by the map's tiles and the atom count), shares of one
+    atom more or less, some empty: within the norm tolerance of the oracle, slabs equal to the map, a sum adds to
+    out."""
+    import torch
+    a = _signed_atoms(n, n + dims[2], 0.5 * dims[0])
+    h, origin = 0.5, (-1.0, 0.5, 2.0)
+    tune = ktt_b200.Tune(block_x=16, block_y=2, z_iterations=16, x_points=2, precision=prec, rsqrt_soft=12)
+    out = torch.full(dims[::-1], float("nan"), device="cuda")
+    ctx.forward_3d(_t(a), dims, h, origin, tune=tune, out=out)
+    assert errors.report(_np(out), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
+    assert torch.equal(ctx.forward_3d_slab(_t(a), dims, h, 48, dims[2], origin, tune=tune), out[48:])
+    base = torch.linspace(-2, 2, out.numel(), device="cuda").reshape(out.shape)
+    acc = base.clone()
+    ctx.forward_3d(_t(a), dims, h, origin, tune=tune, out=acc, accumulate=True)
+    assert torch.equal(acc, base + out)
+
+
+@pytest.mark.parametrize("n", [1, 24, 47, 49, 200])
+@pytest.mark.parametrize("block", [(32, 4), (7, 3), (16, 1), (8, 4)])
+@pytest.mark.parametrize("shape,prec,soft", [((16, 2, 1), ktt_b200.PREC_FP64_MERGE_SHARED, 12),
+                                             ((16, 2, 1), ktt_b200.PREC_FP32, 2)])
+def test_record_tiles_of_one_warp_in_a_batch(ctx, n, block, shape, prec, soft):
+    """Record tiles whose warp runs through all atoms, blocks with a partial warp, grids that overhang a tile by
+    every number of planes: persistent and separate launches bit for bit, within the norm tolerance of the oracle."""
+    import torch
+    tune = ktt_b200.Tune(block_x=block[0], block_y=block[1], z_iterations=shape[0], x_points=shape[1], unroll=shape[2],
+                         precision=prec, rsqrt_soft=soft)
+    mols = [(_signed_atoms(n, n + nz, 18.0), (35 - nz % 3, 11, nz), 0.5, (-1.0, 0.5, 2.0)) for nz in range(1, 36, 3)]
+    batch = ktt_b200.Batch(ctx, [(_t(a), *rest) for a, *rest in mols], tune)
+    batch.run()
+    ctx.synchronize()
+    maps = [out.clone() for out in batch.outputs]
+    for (a, dims, h, origin), out in zip(mols, maps):
+        assert errors.report(_np(out), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
+    for out in batch.outputs:
+        out.zero_()
+    batch.run(ktt_b200.BATCH_SEPARATE)
+    ctx.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(maps, batch.outputs))
+    batch.close()
+
+
+@pytest.mark.parametrize("block", [(64, 1), (7, 3)])
+@pytest.mark.parametrize("shape,soft", [((8, 2, 2), 2), ((8, 2, 1), 0), ((16, 2, 1), 12), ((16, 2, 4), 0)])
+def test_fp32_tiles_on_a_map_too_large_for_the_plain_kernel(ctx, block, shape, soft):
+    """FP32 configurations of 2 x 8 and 2 x 16 points from 64 tiles an SM on run their own tile: within the norm
+    tolerance of the oracle, slabs equal to the map."""
+    import torch
+    dims, h, origin = (223, 224, 209), 0.5, (-1.0, 0.5, 2.0)
+    a = _signed_atoms(37, 3, 100.0)
+    tune = ktt_b200.Tune(block_x=block[0], block_y=block[1], z_iterations=shape[0], x_points=shape[1], unroll=shape[2],
+                         rsqrt_soft=soft)
+    out = torch.full(dims[::-1], float("nan"), device="cuda")
+    ctx.forward_3d(_t(a), dims, h, origin, tune=tune, out=out)
+    assert errors.report(_np(out), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
+    assert torch.equal(ctx.forward_3d_slab(_t(a), dims, h, 96, dims[2], origin, tune=tune), out[96:])
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 300, 1), (131, 3, 9), (129, 7, 17), (257, 2, 8), (96, 33, 5)])
+@pytest.mark.parametrize("tune", [
+    dict(z_iterations=8, x_points=1, unroll=2, rsqrt_soft=2), dict(z_iterations=8, x_points=4, rsqrt_soft=3),
+    dict(z_iterations=16, x_points=1), dict(z_iterations=4, x_points=4),
+    dict(z_iterations=8, x_points=2, precision=ktt_b200.PREC_COMPENSATED),
+    dict(z_iterations=8, x_points=2, precision=ktt_b200.PREC_FP64_MERGE, rsqrt_soft=2)])
+def test_linear_tiles_of_the_one_cta_kernels(ctx, dims, tune):
+    """As test_linear_and_rectangular_tiles, for tiles that run a CTA each on maps of this size: blocks of 64 x 1 and
+    7 x 3 against a block of one thread, bit for bit."""
+    import torch
+    a = _signed_atoms(77, sum(dims), 0.5 * max(dims))
+    h, origin = 0.5, (-1.0, 0.5, 2.0)
+    one = ctx.forward_3d(_t(a), dims, h, origin, tune=ktt_b200.Tune(block_x=1, block_y=1, **tune))
+    assert errors.report(_np(one), oracle.grid3d(a, h, dims, origin))["rel_norm"] <= TOL_NORM
+    for block in ((64, 1), (7, 3)):
+        out = torch.full(dims[::-1], float("nan"), device="cuda")
+        ctx.forward_3d(_t(a), dims, h, origin, tune=ktt_b200.Tune(block_x=block[0], block_y=block[1], **tune), out=out)
+        assert torch.equal(out, one)
