@@ -137,7 +137,10 @@ static cudaError_t launch_batched(coul_batch* b, cudaStream_t stream, int accumu
                   b->ctx->d_status};
     void* args[] = {&p};
     const dim3 block(static_cast<unsigned>(b->tune.block_x), static_cast<unsigned>(b->tune.block_y), 1);
-    return cudaLaunchKernel(b->variant->kernel, dim3(static_cast<unsigned>(b->grid_ctas)), block, args, b->smem, stream);
+    // No more CTAs than items: of a grid of all resident slots the first to arrive took a small batch's items, several
+    // on one SM (2 molecules of 200 .. 400 atoms 86 us, 4 of 200 .. 1,000 152; so 57 and 109).
+    const unsigned ctas = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(b->grid_ctas, b->total_items)));
+    return cudaLaunchKernel(b->variant->kernel, dim3(ctas), block, args, b->smem, stream);
 }
 
 extern "C" {
