@@ -113,8 +113,8 @@ typedef struct coul_tune {
                          the atom-split form also the warps of a block) take turns in 8 / n phases
                          and pair p in phase g is on the FMA pipe when g * n + p < rsqrt_soft.  Either
                          way the share is rsqrt_soft / 8.
-                         10 + k (k = 0..7): a share of (2k + 1) / 16: with n >= 16 that many of every
-                         16 pairs, spread evenly; with fewer, successive patterns alternate between k
+                         10 + k (k = 0..7): a share of (2k + 1) / 16: with n = 16 that many of the
+                         pairs, spread evenly; otherwise successive patterns alternate between k
                          and k + 1 eighths.
                          The FMA-pipe root is good to 4.6e-7 (MUFU: 1.3e-7); tiles of 2 x 16 points with FP64
                          merge, and calls without a configuration, take a longer one, good to 1.1e-7.

@@ -526,16 +526,13 @@ int launch_forward(coul_ctx* ctx, const VariantEntry* v, const FwdParams& prm, i
     }
     L.grid = dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(gz));
     if (v->key.split == 0 && linear_tiles(t->precision, t->z_iterations, mode)) {
-        // linear x-y tiles where they are fewer than the block's rectangles
         const int64_t columns = (prm.nx + t->x_points - 1) / t->x_points;
         const int64_t threads = static_cast<int64_t>(t->block_x) * t->block_y;
         const int64_t tiles = (columns * prm.ny + threads - 1) / threads;
-        if (tiles < gx * gy) {
-            const int64_t rows = (tiles + (int64_t{1} << 30) - 1) >> 30;  // blocks beyond the last tile store nothing
-            L.p.columns = static_cast<int>(columns);
-            L.grid.x = static_cast<unsigned>((tiles + rows - 1) / rows);
-            L.grid.y = static_cast<unsigned>(rows);
-        }
+        const int64_t rows = (tiles + (int64_t{1} << 30) - 1) >> 30;  // blocks beyond the last tile store nothing
+        L.p.columns = static_cast<int>(columns);
+        L.grid.x = static_cast<unsigned>((tiles + rows - 1) / rows);
+        L.grid.y = static_cast<unsigned>(rows);
     }
     L.smem = t->atom_source == COUL_ATOMS_SHARED_TMA
                  ? tile_smem_bytes(t->block_x * t->block_y, t->z_iterations, t->x_points, v->key.soa, t->precision, mode)

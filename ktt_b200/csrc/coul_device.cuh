@@ -51,7 +51,7 @@ struct FwdParams {
     float h, ox, oy, oz;
     float* out;
     int accumulate;
-    int columns;  // 3D, one CTA per tile: columns of x points per row of linear x-y tiles, 0 for the block's rectangles
+    int columns;  // 3D, one CTA per tile: columns of x points per row of linear x-y tiles
     int* status;
 };
 
@@ -307,13 +307,13 @@ constexpr float kSoftFar = 0x1p48f;    // coordinates below this on both sides k
 // slot s = (stage phase) * NP + p for NP < 8, s = p % 8 otherwise, and a slot takes the FMA pipe
 // when s < SOFT.  The share is SOFT / 8 at every tile size.  From kSoftAlternate on
 // (SOFT = kSoftAlternate + k) two such patterns alternate between k and k + 1 soft slots, a share
-// of (2k + 1) / 16; with NP >= 16 that share fits into one pattern, and pair p is soft where
+// of (2k + 1) / 16; with NP = 16 that share fits into one pattern, and pair p is soft where
 // (p + 1) (2k + 1) / 16 passes a whole number: 2k + 1 of every 16 pairs, spread evenly, so that a run of
 // MUFU pairs and a run of FMA-pipe pairs never wait for one another (5/16 of 16 pairs in a bare pair
 // loop: 6.30 Tpair/s spread, 6.05 side by side).  In 2D the whole eighths of NP >= 8 pairs are spread in the
 // same way (a 1024 x 1024 slice x 20,000 atoms with 16 points a thread, 2/8: 3.68 ms, side by side 3.81); in
-// 3D they stay side by side, where the forms with FP64 sums lose 1.5 % by it.  soft_phases is the number of stage phases of one whole
-// pattern.
+// 3D they stay side by side, where the forms with FP64 sums lose 1.5 % by it, and 32 pairs (32 x 2 points) alternate, where
+// spread ones lose 3 to 7 %.  soft_phases is the number of stage phases of one whole pattern.
 constexpr int kSoftAlternate = 10;
 // SOFT = share + kSoftFull: the share's pairs take rsqrt_full, and the charge as it is
 constexpr int kSoftFull = 64;
@@ -322,7 +322,7 @@ constexpr float soft_scale(int soft) { return soft >= kSoftFull ? 1.0f : kSoftRs
 constexpr int soft_group(int np) { return np >= 8 ? 1 : 8 / np; }
 constexpr int soft_phases(int soft, int np)
 {
-    return soft == 0 || np >= 16 ? 1 : (soft_share(soft) >= kSoftAlternate ? 2 : 1) * soft_group(np);
+    return soft == 0 || np == 16 ? 1 : (soft_share(soft) >= kSoftAlternate ? 2 : 1) * soft_group(np);
 }
 constexpr bool spread_soft(int p, int sixteenths) { return (p + 1) * sixteenths / 16 != p * sixteenths / 16; }
 
@@ -344,7 +344,7 @@ __device__ __forceinline__ void with_phase(const int phase, F&& f)
 template <int SOFT, int NP, int PHASE, bool SPREAD>
 __device__ __forceinline__ constexpr bool pair_is_soft(int p)
 {
-    if constexpr (SOFT >= kSoftAlternate && NP >= 16)
+    if constexpr (SOFT >= kSoftAlternate && NP == 16)
         return spread_soft(p, 2 * (SOFT - kSoftAlternate) + 1);
     if constexpr (SPREAD && SOFT < kSoftAlternate && NP >= 8)
         return spread_soft(p & 7, 2 * SOFT);

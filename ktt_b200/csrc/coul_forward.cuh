@@ -690,17 +690,17 @@ constexpr int fwd_min_blocks(const int prec, const int points)
     return prec == kPrecFp64MergeShared ? (points <= 16 ? 5 : points <= 32 ? 2 : 1) : 1;
 }
 
-// The x-y tiles of a 3D map are linear where the block's own rectangles would be padded more: the
-// plane is numbered row by row in columns of XP points (p.columns = ceil(nx / XP) a row) and thread i
-// of plane tile b takes column b * threads + i, so only the plane's last tile and, where XP does not
-// divide nx, a row's last column hold points outside the grid.  A point keeps its position x mod XP in
-// its thread, so its value does not depend on the tile it falls in.  On B200 a 131 x 117 x 125 map
-// (block 64 x 1, two points along x, so rectangles 128 wide) takes 1.95 ms instead of 3.52, and the
-// FP64-pair form on 96^3 (rectangles 256 wide) 4.17 ms instead of 8.14.
+// The x-y tiles of a 3D map are linear: the plane is numbered row by row in columns of XP points
+// (p.columns = ceil(nx / XP) a row) and thread i of plane tile b takes column b * threads + i, so only the
+// plane's last tile and, where XP does not divide nx, a row's last column hold points outside the grid, where the
+// block's own rectangles pad each row and column.  A point keeps its position x mod XP in its thread, so its
+// value does not depend on the tile it falls in.  On B200 a 131 x 117 x 125 map (block 64 x 1, two points along x, so
+// rectangles 128 wide) takes 1.95 ms instead of 3.52.  Rectangles where they are no more would save a division, but
+// the second way of placing a tile costs some pair loops registers: FP32 sums of 8 x 4 points with 2/8 on 128^3 x
+// 2,000 926 us with rectangles alone, 1,002 with both, 933 so.
 constexpr bool linear_tiles(const int prec, const int zi, const int mode)
 {
-    // not the small shared-sum tiles: at their 48 registers the second way of placing a tile costs the
-    // pair loop 0.6 % (256^3 x 65,536: 197.0 against 195.9 ms), whichever of the two a launch takes
+    // not the small shared-sum tiles, whose 48 registers are all in use (256^3 x 65,536: 197.0 against 195.9 ms)
     return mode == kModeGrid3d && (prec != kPrecFp64MergeShared || zi >= 16);
 }
 
@@ -709,7 +709,13 @@ template <int ZI, int XP, int UNR, int SRC, int SOA, int PREC, int SOFT, int MOD
 __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) fwd_kernel(const FwdParams p, const int vec_ok)
 {
     int x0, yrow, z0;
-    if constexpr (MODE == kModeGrid3d) {
+    if constexpr (linear_tiles(PREC, ZI, MODE)) {
+        const int64_t tile = static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
+        const int64_t column = tile * (blockDim.x * blockDim.y) + threadIdx.y * blockDim.x + threadIdx.x;
+        yrow = static_cast<int>(column / p.columns);
+        x0 = static_cast<int>(column % p.columns) * XP;
+        z0 = p.z_base + static_cast<int>(blockIdx.z) * ZI;
+    } else if constexpr (MODE == kModeGrid3d) {
         x0 = (blockIdx.x * blockDim.x + threadIdx.x) * XP;
         yrow = blockIdx.y * blockDim.y + threadIdx.y;
         z0 = p.z_base + static_cast<int>(blockIdx.z) * ZI;
@@ -717,14 +723,6 @@ __global__ void __launch_bounds__(kMaxThreads, fwd_min_blocks(PREC, XP * ZI)) fw
         x0 = (blockIdx.x * blockDim.x + threadIdx.x) * XP;
         yrow = (blockIdx.y * blockDim.y + threadIdx.y) * ZI;
         z0 = 0;
-    }
-    if constexpr (linear_tiles(PREC, ZI, MODE)) {
-        if (p.columns > 0) {
-            const int64_t tile = static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
-            const int64_t column = tile * (blockDim.x * blockDim.y) + threadIdx.y * blockDim.x + threadIdx.x;
-            yrow = static_cast<int>(column / p.columns);
-            x0 = static_cast<int>(column % p.columns) * XP;
-        }
     }
     uint32_t gstage = 0;
     if constexpr (record_tile(ZI, XP, SRC, SOA, PREC, MODE)) {
