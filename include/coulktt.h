@@ -80,7 +80,8 @@ enum {
 /* Precision form.  FP32, compensated and both FP64 merges evaluate each pair in FP32 and differ in
    how they accumulate; FP64 pairs evaluates each pair in FP64. */
 enum {
-    COUL_PREC_FP32 = 0,        /* one FP32 accumulator per point (KTT's kernel) */
+    COUL_PREC_FP32 = 0,        /* one FP32 accumulator per point (KTT's kernel); where the atoms of a tile are
+                                  split (atom_split, coul_tune_launched), one per part, added in order */
     COUL_PREC_COMPENSATED = 1, /* FP32 partial per 64-atom sub-tile, merged by two-sum into (sum, error) */
     COUL_PREC_FP64_MERGE = 2,  /* FP32 partial per 64-atom sub-tile, merged into an FP64 accumulator */
     COUL_PREC_FP64_PAIRS = 3,  /* every pair in FP64: exact differences, FP64 r^2, MUFU rsqrt estimate
@@ -97,7 +98,8 @@ enum {
  * map onto each field.
  */
 typedef struct coul_tune {
-    int block_x;      /* threads per block along x             [WORK_GROUP_SIZE_X] */
+    int block_x;      /* threads per block along x             [WORK_GROUP_SIZE_X]; some kernels bring their own
+                         block: coul_tune_launched */
     int block_y;      /* threads per block along y             [WORK_GROUP_SIZE_Y] */
     int z_iterations; /* grid points per thread along z         [Z_ITERATIONS] (3D); along y for 2D */
     int x_points;     /* grid points per thread along x, stored as one float/float2/float4 vector
@@ -218,6 +220,18 @@ COUL_API void coul_tune_default(coul_tune* tune);
 COUL_API int coul_tune_supported(const coul_tune* tune);
 /* The same check for coul_forward_2d (2D-slice variants). */
 COUL_API int coul_tune_supported_2d(const coul_tune* tune);
+/*
+ * The configuration that a launch of `tune` over the whole grid runs (float4 atoms).  It is `tune` itself except where
+ * a kernel with its own block takes the place of a configuration's, whatever its block and unrolling:
+ *   FP32 sums of 2 x 8 and 2 x 16 points a thread on maps of fewer than 64 tiles (32 columns of two points by 16
+ *     planes) an SM: the kernel of calls without a configuration (csrc/coul_plain.cu), with the configuration's share of
+ *     FMA-pipe roots, a tile's atoms split over its warps;
+ *   FP64 merge of 2 x 16 points a thread, where the atoms are split (csrc/coul_forward.cuh, record_split_kernel);
+ *   FP64 pairs: tiles of 32 columns of threads, of 8 x 2 points where the configuration has more than 16 a thread.
+ * Configurations with the same answer are one launch, so that a search need time only one of them.
+ */
+COUL_API int coul_tune_launched(coul_ctx* ctx, const coul_tune* tune, const coul_grid* grid, int64_t n_atoms,
+                                coul_tune* launched);
 /* Number of compiled forward variants, and the i-th one (for the tuner's space checks): its
    tuning fields (block shape left at the default), whether it is a 2D-slice variant, and whether
    it reads the four-array atom layout. */

@@ -130,6 +130,7 @@ def load_library():
         "coul_elapsed_ms": [vp, ctypes.POINTER(ctypes.c_double)],
         "coul_tune_supported": [T],
         "coul_tune_supported_2d": [T],
+        "coul_tune_launched": [vp, T, G, i64, T],
         "coul_batch_tune_supported": [T],
         "coul_variant_count": [],
         "coul_variant_get": [ci, T, ctypes.POINTER(ci), ctypes.POINTER(ci)],
@@ -293,6 +294,13 @@ class CoulombContext:
         if tuple(out.shape) != tuple(shape) or out.dtype != torch.float32 or not out.is_contiguous():
             raise CoulombError(COUL_ERR_INVALID_ARGUMENT, f"out must be a contiguous float32 tensor of shape {shape}")
         return out
+
+    def launched_tune(self, tune: Tune, dims, n_atoms: int) -> Tune:
+        """The configuration that forward_3d with `tune` runs on a map of these dims (coul_tune_launched)."""
+        g, out = _grid(dims, 1.0, None), _Tune()
+        _check(self._lib.coul_tune_launched(self._ctx, ctypes.byref(tune.c()), ctypes.byref(g), int(n_atoms),
+                                            ctypes.byref(out)))
+        return Tune(*(getattr(out, name) for name, _ in _Tune._fields_))
 
     # -- forward ------------------------------------------------------------------------------
     def forward_3d(self, atoms, dims, spacing, origin=None, tune: Tune | None = None, out=None,

@@ -9,7 +9,8 @@
 The kernel is registered with the ktt:: tuner exactly as a KTT host program registers
 directCoulombSum (Examples/CoulombSum3d/CoulombSum3d.cpp:100-237) -- definition, arguments, tuning
 parameters with thread modifiers and constraints -- with the B200 parameters added (X_POINTS,
-RSQRT_SOFT) and a constraint that keeps the search inside the compiled variants; the batched map is
+RSQRT_SOFT), a constraint that keeps the search inside the compiled variants and one that keeps a single
+configuration of those that run as one launch; the batched map is
 the tuner's "coulombBatch" definition.  KTT's searchers pick the configurations (MCMC by default,
 Examples' ConfigurationCount budget), every configuration is validated by the tuner against a
 reference computation registered through Tuner::SetReferenceComputation (Source/Tuner.h:610;
@@ -23,6 +24,7 @@ differences, square root and division), which shares no arithmetic with the tune
 from __future__ import annotations
 
 import argparse
+import itertools
 import json
 import os
 
@@ -62,9 +64,10 @@ def _tune_from(values, names):
                          precision=v.get("PRECISION", 0))
 
 
-def _add_space(ktt, tuner, kernel, definition, space, supported, precisions=(0,)):
+def _add_space(ktt, tuner, kernel, definition, space, supported, precisions=(0,), launched=None):
     """The space's parameters, PRECISION (the accumulation forms searched), KTT's thread modifiers and
-    the constraints."""
+    the constraints.  launched(tune) -> the configuration that runs: of those that run as one launch, the first
+    stays."""
     space = dict(space, PRECISION=list(precisions))
     names = list(space)
     for name, values in space.items():
@@ -78,6 +81,19 @@ def _add_space(ktt, tuner, kernel, definition, space, supported, precisions=(0,)
     tuner.AddConstraint(kernel, ["WORK_GROUP_SIZE_X", "WORK_GROUP_SIZE_Y"], lambda v: 32 <= v[0] * v[1] <= 256)
     # stay inside the compiled variants (a configuration outside them would only report CompilationFailed)
     tuner.AddConstraint(kernel, names, lambda v: supported(_tune_from(v, names)))
+    if launched is not None:
+        first = _first_of_each_launch(space, supported, launched)
+        tuner.AddConstraint(kernel, names, lambda v: tuple(int(x) for x in v) in first)
+
+
+def _first_of_each_launch(space, supported, launched):
+    """The first configuration of the constrained space for each launch."""
+    names, first = list(space), {}
+    for values in itertools.product(*space.values()):
+        tune = _tune_from(values, names)
+        if 32 <= tune.block_x * tune.block_y <= 256 and supported(tune):
+            first.setdefault(tuple(launched(tune).as_dict().values()), values)
+    return set(first.values())
 
 
 SEARCHERS = ["mcmc", "random", "deterministic", "profile"]
@@ -161,9 +177,12 @@ def tune_map3d(grid: int = 256, atoms: int = 65536, searcher: str = "mcmc", budg
     tuner.SetGlobalSizeType(ktt.GlobalSizeType.CUDA)
     definition = tuner.AddKernelDefinition("directCoulombSum", "", ktt.DimensionVector(g, g, g), ktt.DimensionVector())
     kernel = tuner.CreateSimpleKernel("CoulombSum", definition)
-    _add_space(ktt, tuner, kernel, definition, MAP3D_SPACE, ktt_b200.tune_supported, precisions)
+    ctx = None if dry_run else ktt_b200.CoulombContext(0)
+    _add_space(ktt, tuner, kernel, definition, MAP3D_SPACE, ktt_b200.tune_supported, precisions,
+               launched=None if dry_run else lambda tune: ctx.launched_tune(tune, w.dims, n))
     if dry_run:
         return {"configurations": tuner.GetConfigurationsCount(kernel)}
+    ctx.close()
 
     ro = ktt.ArgumentAccessType.ReadOnly
     arg_ids = [tuner.AddArgumentVectorFloat(w.atoms.reshape(-1), ro)]

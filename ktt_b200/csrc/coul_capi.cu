@@ -841,6 +841,46 @@ COUL_API int coul_tune_supported(const coul_tune* t) { return validate_tune(t, k
 
 COUL_API int coul_tune_supported_2d(const coul_tune* t) { return validate_tune(t, kModeSlice2d, 0, nullptr); }
 
+COUL_API int coul_tune_launched(coul_ctx* ctx, const coul_tune* tune, const coul_grid* grid, int64_t n_atoms,
+                                coul_tune* launched)
+{
+    if (ctx == nullptr || launched == nullptr || n_atoms < 0)
+        return set_error(COUL_ERR_INVALID_ARGUMENT, "ctx or output is NULL, or the atom count negative");
+    const VariantEntry* v = nullptr;
+    int rc = validate_grid(grid);
+    if (rc || (rc = validate_tune(tune, kModeGrid3d, 0, &v)))
+        return rc;
+    FwdLaunch L{};
+    L.p.nx = grid->nx;
+    L.p.ny = grid->ny;
+    L.p.nz = grid->nz;
+    L.p.n_atoms = n_atoms;
+    *launched = *tune;
+    launched->unroll = v->key.unroll;
+    const auto warps = [&] {  // kernels of 256 threads in linear tiles, whatever the configuration's block
+        launched->block_x = 32 * kRecordSplitWarps;
+        launched->block_y = 1;
+    };
+    if (plain_tile(ctx, v, tune, kModeGrid3d, L.p, grid->nz)) {
+        warps();
+        launched->z_iterations = 16;
+        launched->unroll = 1;
+    } else if (tune->precision == COUL_PREC_FP64_PAIRS) {
+        warps();
+        launched->z_iterations = fp64_zi(tune->z_iterations, tune->x_points);
+        launched->x_points = fp64_xp(tune->z_iterations, tune->x_points);
+    } else if (v->key.split == 0 && tune->precision != COUL_PREC_FP32 &&
+               record_tile(tune->z_iterations, tune->x_points, tune->atom_source, v->key.soa, tune->precision, kModeGrid3d)) {
+        record_split_setup(ctx, L, tune, grid->nz);
+        if (L.record_group > 0) {
+            warps();
+            launched->unroll = 1;
+            launched->precision = COUL_PREC_FP64_MERGE_SHARED;
+        }
+    }
+    return COUL_OK;
+}
+
 COUL_API int coul_variant_count(void) { return static_cast<int>(registry().size()); }
 
 COUL_API int coul_variant_get(int i, coul_tune* t, int* is_2d, int* is_soa)

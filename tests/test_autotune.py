@@ -158,3 +158,37 @@ def test_full_map3d_search_validated_against_the_oracle():
         json.dump(result, f, indent=1)
         f.write("\n")
     assert ktt_b200.tune_supported(ktt_b200.Tune(**result["tune"]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grid,n", [(64, 300), (256, 3000)])
+def test_search_space_holds_each_launch_once(grid, n):
+    """Configurations that run as one launch (a kernel with its own block in their place) are one configuration of the
+    search, equal in their maps bit for bit; the others stay."""
+    import torch
+    dims = (grid,) * 3
+    space = dict(autotune.MAP3D_SPACE, PRECISION=[0, 2, 4])
+    names = list(space)
+    ctx = ktt_b200.CoulombContext(0)
+    try:
+        first = autotune._first_of_each_launch(space, ktt_b200.tune_supported, lambda t: ctx.launched_tune(t, dims, n))
+        kept = [autotune._tune_from(v, names) for v in first]
+        launched = [tuple(ctx.launched_tune(t, dims, n).as_dict().values()) for t in kept]
+        assert len(set(launched)) == len(launched)
+        # an FP32 tile of 8 x 1 points runs as itself at any block
+        assert sum(t.precision == 0 and t.z_iterations == 8 and t.x_points == 1 and t.rsqrt_soft == 2 and t.unroll == 1
+                   for t in kept) > 5
+        # 2 x 16 points with FP64 merge: one for each share, and with FP32 sums on the small map
+        for precision in ((0, 2) if grid == 64 else (2,)):
+            same = [t for t in kept if t.z_iterations == 16 and t.x_points == 2 and t.rsqrt_soft == 2
+                    and t.precision in ((0,) if precision == 0 else (2, 4))]
+            assert len(same) <= 1
+        if grid == 64:
+            rng = np.random.default_rng(0)
+            atoms = torch.from_numpy(rng.uniform(0.0, 32.0, (n, 4)).astype(np.float32)).cuda()
+            for fields in (dict(z_iterations=8, rsqrt_soft=2), dict(z_iterations=16, rsqrt_soft=12, precision=2)):
+                a, b = (ktt_b200.Tune(block_x=x, block_y=y, x_points=2, **fields) for x, y in ((64, 1), (16, 4)))
+                assert ctx.launched_tune(a, dims, n) == ctx.launched_tune(b, dims, n)
+                assert torch.equal(ctx.forward_3d(atoms, dims, 0.5, tune=a), ctx.forward_3d(atoms, dims, 0.5, tune=b))
+    finally:
+        ctx.close()
