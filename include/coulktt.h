@@ -74,7 +74,8 @@ typedef enum coul_status {
 /* Where the atom stream is read from inside the kernel (KTT USE_CONSTANT_MEMORY). */
 enum {
     COUL_ATOMS_SHARED_TMA = 0, /* tiles staged into shared memory by TMA bulk copies */
-    COUL_ATOMS_CONSTANT = 1    /* chunks of 4096 atoms copied into __constant__ memory */
+    COUL_ATOMS_CONSTANT = 1    /* chunks of 4096 atoms copied into __constant__ memory, one bank per CUDA
+                                  context: launches of this form on one stream at a time */
 };
 
 /* Precision form.  FP32, compensated and both FP64 merges evaluate each pair in FP32 and differ in
