@@ -175,11 +175,35 @@ __device__ __forceinline__ bool soft_axis(const int count, const float h, const 
     return fabsf(origin) < kSoftFar && fabsf(fmaf(static_cast<float>(count), h, origin)) < kSoftFar;
 }
 
-// Whether every r^2 of an atom and a 3D tile is within that range, from the atom's place in x and y and its
-// smallest and largest |dz| to the tile's planes (the grid's own x and y are soft_axis').
-__device__ __forceinline__ bool soft_atom(const float4 a, const float dz_min, const float dz_max)
+// Whether an atom's place in x and y and its largest |dz| to a tile's planes are within it (the grid's own x and y
+// are soft_axis').
+__device__ __forceinline__ bool soft_place(const float4 a, const float dz_max)
 {
-    return fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && dz_min >= kSoftNear && dz_max < kSoftFar;
+    return fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && dz_max < kSoftFar;
+}
+
+// Whether one of a warp's `count` staged atoms (x, y first, `stride` float4 apart) lies on one of its lanes' columns,
+// XN points along x by YN along y.  Asked where an atom lies in a plane of the tile, so that of atoms that all do (a
+// lattice, a slab, 128^3 x 2,000 by the tuned configuration) each sends its own tile's batches through MUFU, not those
+// of every tile between its planes.
+template <int XN, int YN>
+__device__ __forceinline__ bool on_columns(const uint32_t lanes, const float4* rec, const int stride, const int count,
+                                           const float (&gx)[XN], const float (&gy)[YN])
+{
+    bool hit = false;
+#pragma unroll 4
+    for (int j = 0; j < count; ++j) {
+        const float4 a = rec[j * stride];
+        bool x = false, y = false;
+#pragma unroll
+        for (int k = 0; k < XN; ++k)
+            x = x || !(fabsf(gx[k] - a.x) >= kSoftNear);
+#pragma unroll
+        for (int k = 0; k < YN; ++k)
+            y = y || !(fabsf(gy[k] - a.y) >= kSoftNear);
+        hit = hit || (x && y);
+    }
+    return __any_sync(lanes, hit);
 }
 
 __device__ __forceinline__ void dz_range(const float4 dz, float& dz_min, float& dz_max)
@@ -239,7 +263,7 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
     for (int64_t b = a0; b < a1; b += kRecordAtoms) {
         const int count = static_cast<int>(a1 - b < kRecordAtoms ? a1 - b : kRecordAtoms);
         __syncwarp();  // the previous records have been read
-        bool inside = soft_grid;
+        bool ok = soft_grid, near = false;
         for (int j = lane; j < count; j += lanes) {
             const float4 a = j == lane ? next : p.atoms[b + j];
             float4* r = rec + j * (record_floats(ZI) / 4);
@@ -252,10 +276,16 @@ __device__ __forceinline__ void record_range(const FwdParams& p, float4* rec, co
                 r[1 + m] = dz;
                 dz_range(dz, dz_min, dz_max);
             }
-            inside = inside && soft_atom(a, dz_min, dz_max);
+            ok = ok && soft_place(a, dz_max);
+            near = near || !(dz_min >= kSoftNear);
         }
-        const bool soft = SOFT == 0 || __all_sync(0xffffffffu >> (32 - lanes), inside);
+        const uint32_t warp_lanes = 0xffffffffu >> (32 - lanes);
+        bool soft = SOFT == 0 || __all_sync(warp_lanes, ok && !near);
         __syncwarp();
+        if (SOFT != 0 && !soft && __all_sync(warp_lanes, ok)) {
+            const float y[1] = {gy};
+            soft = !on_columns(warp_lanes, rec, record_floats(ZI) / 4, count, gx, y);
+        }
         if (lane < kRecordAtoms && b + kRecordAtoms + lane < a1)
             next = p.atoms[b + kRecordAtoms + lane];
         if (!soft)

@@ -204,8 +204,13 @@ __global__ void __launch_bounds__(kPlainThreads, 2) plain_3d_kernel(const PlainP
             if (4 * m < p.depth)
                 dz_range(dz, dz_min, dz_max);
         }
-        const bool soft = SOFT != 0 && __all_sync(0xffffffffu, lane >= cnt || (soft_grid && soft_atom(a, dz_min, dz_max)));
+        const bool ok = lane >= cnt || (soft_grid && soft_place(a, dz_max));
+        bool soft = SOFT != 0 && __all_sync(0xffffffffu, ok && (lane >= cnt || dz_min >= kSoftNear));
         __syncwarp();
+        if (SOFT != 0 && !soft && __all_sync(0xffffffffu, ok)) {
+            const float y[1] = {gy};
+            soft = !on_columns(0xffffffffu, rec, kPlainRecord / 4, cnt, gx, y);
+        }
         if (b + 32 + lane < end)
             a = p.f.atoms[b + 32 + lane];
         // a tile that overhangs the grid by half or more evaluates its first half
@@ -275,10 +280,17 @@ __global__ void __launch_bounds__(kPlainThreads, 4) plain_2d_kernel(const PlainP
         __syncwarp();
         rec[lane] = a;
         // an atom's .z is its dz^2 to the slice
-        const bool inside = fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && a.z >= kSoftNear * kSoftNear &&
-                            a.z < kSoftFar * kSoftFar;
-        const bool soft = SOFT != 0 && __all_sync(0xffffffffu, lane >= cnt || (soft_grid && inside));
+        const bool ok = lane >= cnt || (soft_grid && fabsf(a.x) < kSoftFar && fabsf(a.y) < kSoftFar && a.z >= 0.0f &&
+                                        a.z < kSoftFar * kSoftFar);
+        bool soft = SOFT != 0 && __all_sync(0xffffffffu, ok && (lane >= cnt || a.z >= kSoftNear * kSoftNear));
         __syncwarp();
+        if (SOFT != 0 && !soft && __all_sync(0xffffffffu, ok)) {
+            float y[kPlain2dY];
+#pragma unroll
+            for (int m = 0; m < kPlain2dY; ++m)
+                y[m] = coul::lane(gy[m / 2], m & 1);
+            soft = !on_columns(0xffffffffu, rec, 1, cnt, gx, y);
+        }
         if (b + 32 + lane < end)
             a = p.f.atoms[b + 32 + lane];
         if (soft) {

@@ -229,3 +229,41 @@ def test_root_of_one_pair_at_mufu_precision(ctx, fields):
             maps.append(ctx.forward_2d(_cuda(flat), h, dims[0], dims[1]).cpu().numpy())
         for v in maps:
             assert np.max(np.abs(v / (exact if v.ndim == 3 else exact[0]) - 1)) <= 2.0**-22.9 + 2.0**-30
+
+
+@pytest.mark.parametrize("h,origin", [(0.5, (-7.25, 3.0, 1e3)), (0.01, (1e6, -1e6, 1e6)), (0.01, (0.0, 3e4, 0.0)),
+                                      (2.0**-44, (0.0, 0.0, 0.0)), (-0.5, (9.0, 9.0, 9.0)), (1e3, (-2e4, 0.0, 1e5))])
+@pytest.mark.parametrize("dims", [(40, 9, 16), (97, 40, 33)])
+@pytest.mark.parametrize("fields", [None, dict(z_iterations=16, x_points=2, rsqrt_soft=12, precision=4)])
+def test_atoms_on_points_of_fine_and_far_grids(ctx, h, origin, dims, fields):
+    """Eight charges of 1 on grid points among 600 atoms, some of them in a plane or a column of the grid: +inf at every
+    point whose FP32 coordinates equal a charge's (several, where the spacing is finer than the origin's rounding), the
+    oracle's value elsewhere."""
+    rng = np.random.default_rng(dims[0])
+    g = [(np.arange(d) * np.float64(np.float32(h)) + np.float64(np.float32(o))).astype(np.float32)
+         for d, o in zip(dims, origin)]
+    lo = np.array([min(x[0], x[-1]) for x in g], dtype=np.float64)
+    hi = np.array([max(x[0], x[-1]) for x in g], dtype=np.float64)
+    a = np.zeros((600, 4), dtype=np.float32)
+    a[:, :3] = lo + (hi - lo) * rng.uniform(-0.3, 1.3, (600, 3))
+    a[:, 3] = rng.uniform(-1.0, 1.0, 600)
+    for j in range(100):  # in one or two of a point's coordinates
+        for c in ((2,), (0, 1), (1, 2), (0, 2))[j % 4]:
+            a[j, c] = rng.choice(g[c])
+    a[600 - 8:, :3] = np.stack([rng.choice(x, 8) for x in g], 1)
+    a[600 - 8:, 3] = 1.0
+    tune = ktt_b200.Tune(block_x=16, block_y=2, **fields) if fields else None
+    out = ctx.forward_3d(_cuda(a), dims, h, origin, tune=tune).cpu().numpy()
+    hit = np.zeros(dims[::-1], dtype=bool)
+    for x, y, z, q in a:
+        hit |= (g[2] == z)[:, None, None] & (g[1] == y)[None, :, None] & (g[0] == x)[None, None, :]
+    assert hit.any()
+    plus = np.zeros(dims[::-1], dtype=bool)
+    for x, y, z, q in a[600 - 8:]:
+        plus |= (g[2] == z)[:, None, None] & (g[1] == y)[None, :, None] & (g[0] == x)[None, None, :]
+    only = plus & np.isposinf(out)
+    assert np.array_equal(only, plus) or (hit & ~plus).any()
+    assert np.all(np.isfinite(out[~hit]))
+    with np.errstate(divide="ignore", invalid="ignore"):
+        ref = oracle.grid3d(a, h, dims, origin)
+    assert np.linalg.norm(out[~hit] - ref[~hit]) <= TOL * np.linalg.norm(ref[~hit])
