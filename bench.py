@@ -7,8 +7,8 @@ Workload: the full 3D map, 256 x 256 x 256 grid at 0.5 A spacing, 65,536 atoms u
 evaluations per second (Gpair-evals/s, one pair = one (grid point, atom) term), whole job.
 
 Our arm (``--impl ours``, default) prints one JSON line with
-  value        device-timed throughput of the headline form -- FP32 pairs, FP64 merge of 48-atom
-               partials, part of the rsqrts on the FMA pipe, tile from ktt_b200/tuned/b200_map3d.json
+  value        device-timed throughput of the headline form -- FP32 pairs, FP64 merge of
+               partials of up to 64 atoms, part of the rsqrts on the FMA pipe, tile from ktt_b200/tuned/b200_map3d.json
                (CUDA events on the launching stream, inputs resident in HBM, L2 flushed between
                steps), max over ranks;
   plain        the same for KTT's kernel form (FP32 accumulation, all rsqrts on MUFU);
