@@ -325,8 +325,9 @@ COUL_API int coul_forward_3d_host_plain(coul_ctx* ctx, const float* h_atoms, int
  * least-squares loss L = 0.5 sum_i w_i (V_i - T_i)^2 pass G_i = w_i (V_i - T_i).  No counterpart in KTT
  * (it tunes forward kernels only); the PyTorch binding wraps forward + adjoint as an autograd function.
  * Asynchronous on the context's stream; keeps an FP64 workspace of 32 * n_atoms * chunks bytes in the
- * context (chunks <= 40 * SMs / atom tiles of 128), which calls on several streams use in turn.  Under stream
- * capture the call's workspace is the graph's own; the context keeps it, for a later capture once the graph is gone.
+ * context (chunks <= 48 * SMs / atom tiles of 128), which calls on several streams use in turn.  Under stream
+ * capture the call's workspace is the graph's own; the context keeps it, for a later capture once the graph is gone,
+ * and has to outlive the graph.
  */
 COUL_API int coul_adjoint_3d(coul_ctx* ctx, const float* d_atoms, int64_t n_atoms, const coul_grid* grid,
                              const float* d_grad_map, float* d_grad_q, float* d_grad_xyz);
